@@ -21,7 +21,7 @@ OUT="$HERE/_ref"
 SRC="${GBSW_REFERENCE_DIR:-$(cd "$HERE/../.." && pwd)/reference}"
 NVCC="${NVCC:-nvcc}"
 mkdir -p "$OUT/src" "$OUT/obj"
-if [ -d "$SRC" ]; then
+if [ -f "$SRC/kernel.cpp" ]; then
   for f in alignments.cpp alignments.hpp driver.cpp driver.hpp kernel.cpp kernel.hpp utils.cpp utils.hpp; do
     cp -f "$SRC/$f" "$OUT/src/$f"
     chmod u+w "$OUT/src/$f"
