@@ -198,6 +198,34 @@ __host__ __device__ __forceinline__ int reverse_band(int a, int b, int na, int n
     return band < (1 << 30) ? (int)band : -1;
 }
 
+// Reverse pass: the band's other side.  An alignment as in reverse_band starts
+// at row r0 and uses at most nrows rows, r0 - 1 of them not at all and gS facing
+// a gap, so m <= nrows - (r0 - 1) - gS and
+//   target <= match * m <= match * (nrows - (r0 - 1) - gS).
+// At any of its cells r - c = (r0 - 1) + gS' - gL' <= (r0 - 1) + gS, so
+//   r <= c + (match * nrows - target) / match:
+// a strip whose last column is l needs only its rows r <= l + that.  Rows past
+// the left neighbour's last one enter a strip from the zero state, as do the
+// rows above its first one, with the same argument.  Returns -1 where
+// reverse_band does.
+__host__ __device__ __forceinline__ int reverse_low_band(int a, int b, int na, int nb, int target, int match,
+                                                         int rev_p) {
+    const int nrows = na < nb ? na : nb;
+    if (rev_p <= 0 || match <= 0 || (a < b) != (na < nb)) return -1;
+    const long long slack = (long long)match * nrows - target;
+    if (slack < 0) return -1;  // inconsistent ends: the pass's own checks report them
+    return (int)(slack / match);
+}
+
+// Last row a reverse strip whose last (1-based) column is `last_col` must
+// compute under `low` (reverse_low_band; -1: nrows).  Even unless it is nrows:
+// the strip-boundary copies move rows (odd, even) together.
+__host__ __device__ __forceinline__ int band_last_row(int last_col, int low, int nrows) {
+    if (low < 0) return nrows;
+    const int r = last_col + low;
+    return r + (r & 1) < nrows ? r + (r & 1) : nrows;
+}
+
 // First row a reverse strip whose first (1-based) column is `first_col` must
 // compute under `band` (reverse_band; -1: row 1).  The band's first row there is
 // first_col - band; the strip starts one row above it, rounded down to an odd

@@ -44,8 +44,12 @@
 //   E'  = max(E + max(ext, open), T, 0)          (= max(E + ext, Ho, 0))
 // which is the int32 kernel's recurrence (see sw_pass.cuh) evaluated per half.
 // Argmax rules and the transposed reverse pass are also the int32 kernel's,
-// band included (reverse_band): a unit's strips start at the rows its wider
-// band needs (unit_band), and both halves compute every row from there.
+// band included (reverse_band, reverse_low_band): a unit's strips start and end
+// at the rows its wider band needs (unit_band, unit_low_band), and both halves
+// compute every row between.  The lower side (strips end at their last column's
+// row) took the mixed DNA batch's reverse pass from 32.9 to 24.4 ms (long pairs,
+// 16 lanes) and the throughput batch's from 2.05 to 1.97 ms (its 20% unrelated
+// pairs have no band to speak of and set the pass's end).
 #include <type_traits>
 
 #include "sw_common.cuh"
@@ -148,6 +152,7 @@ struct Half {
     int nrows, ncols, pad;
     int ncols_run;           // columns computed (reverse: bounded, see reverse_columns)
     int band;                // reverse: the band of reverse_band (-1: every row), until the unit's is set
+    int low;                 // reverse: its other side, reverse_low_band
     bool a_short;
     int target;              // reverse: the forward score
 };
@@ -159,6 +164,13 @@ __device__ __forceinline__ int unit_band(const Half& a, const Half& b) {
     const bool has_a = a.nrows > 0, has_b = b.nrows > 0;
     if ((has_a && a.band < 0) || (has_b && b.band < 0)) return -1;
     return max(has_a ? a.band + a.pad : 0, has_b ? b.band + b.pad : 0);
+}
+
+// The same for the band's other side (reverse_low_band).
+__device__ __forceinline__ int unit_low_band(const Half& a, const Half& b) {
+    const bool has_a = a.nrows > 0, has_b = b.nrows > 0;
+    if ((has_a && a.low < 0) || (has_b && b.low < 0)) return -1;
+    return max(has_a ? a.low : 0, has_b ? b.low : 0);
 }
 
 // Bytes of dynamic shared memory of a protein dual block: both pairs' strip
@@ -207,9 +219,10 @@ __global__ void __launch_bounds__(kThreads, AA ? GBSW_DUAL_MIN_BLOCKS
     constexpr bool kSaveHit = REVERSE && (AA || G <= GBSW_REV_SAVE_HIT_MAX_G);
     __shared__ __align__(16) int4 ssave[(REVERSE && !kSaveHit) ? 1 : 2][C / 4][kThreads];
     __shared__ __align__(16) int2 sbnd[kThreads / G][2][kChunkD];
-    // reverse: the unit's band (unit_band), read at strip set-up only, so kept
-    // out of the registers the row steps need; one slot per thread
-    __shared__ int sband[REVERSE ? kThreads : 1];
+    // reverse: the unit's band (unit_band, unit_low_band), read at strip set-up
+    // and by lane 0 once a chunk, so kept out of the registers the row steps
+    // need; one slot per thread
+    __shared__ int2 sband[REVERSE ? kThreads : 1];
     // DNA reverse: column profiles of this lane's C columns, both pairs: entry k
     // holds {A[2k], B[2k], A[2k+1], B[2k+1]}; a thread reads only its own slice
     // (the forward kernels keep them in registers, preg)
@@ -391,13 +404,17 @@ __global__ void __launch_bounds__(kThreads, AA ? GBSW_DUAL_MIN_BLOCKS
         return cw;
     };
     // Lane 0 starts the copy of the boundary entries of rows [r0, r0 + kChunkD).
+    // Reverse: rows past the previous strip's last one read the zero state.
     auto fetch_chunk = [&](int r0, int buf) {
         if (strip > 0) {
+            const int have = REVERSE ? band_last_row(strip * W, sband[REVERSE ? threadIdx.x : 0].y, nrows) : nrows;
 #pragma unroll
             for (int u = 0; u < kChunkD; u += 2) {
-                if (r0 + u <= nrows) {  // rows r0+u-1, r0+u: 16 bytes inside the buffer
+                if (r0 + u <= have) {  // rows r0+u-1, r0+u: 16 bytes inside the buffer
                     const unsigned dst = (unsigned)__cvta_generic_to_shared(sb + buf * kChunkD + u);
                     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(bnd + (r0 + u - 1)));
+                } else if (REVERSE) {
+                    sb[buf * kChunkD + u] = sb[buf * kChunkD + u + 1] = make_int2((int)open2, 0);
                 }
             }
         }
@@ -472,9 +489,13 @@ __global__ void __launch_bounds__(kThreads, AA ? GBSW_DUAL_MIN_BLOCKS
         mA = mB = 0;
         miA = miB = 0;
         st = 0;
-        // reverse: the strip's steps start at its band's first row
-        if constexpr (REVERSE) st = band_first_row(strip * W + 1, sband[threadIdx.x]) - 1;
         nsteps = nrows + G - 1;
+        if constexpr (REVERSE) {
+            // the strip's steps start at its band's first row and end at its last one
+            const int2 band = sband[threadIdx.x];
+            st = band_first_row(strip * W + 1, band.x) - 1;
+            nsteps = band_last_row(strip * W + W, band.y, nrows) + G - 1;
+        }
         codes = fetch_codes(st, codesB);
         if constexpr (kSplitCodes) issue_window(st + kChunkD);
         else codes_next = fetch_codes(st + kChunkD, codesB_next);
@@ -494,7 +515,7 @@ __global__ void __launch_bounds__(kThreads, AA ? GBSW_DUAL_MIN_BLOCKS
         hh.rowseq = hh.colseq = p.ref;
         hh.a_short = false;
         hh.target = 0;
-        hh.band = -1;
+        hh.band = hh.low = -1;
         if (pid < 0) return;
         const int64_t ra = p.ref_off[pid], rb = p.ref_off[pid + 1];
         const int64_t qa = p.query_off[pid], qb = p.query_off[pid + 1];
@@ -531,6 +552,7 @@ __global__ void __launch_bounds__(kThreads, AA ? GBSW_DUAL_MIN_BLOCKS
             hh.ncols = hh.a_short ? nb : na;
             hh.ncols_run = reverse_columns(a, b, na, nb, hh.target, p.match, p.rev_p);
             hh.band = reverse_band(a, b, na, nb, hh.target, p.match, p.rev_p);
+            hh.low = reverse_low_band(a, b, na, nb, hh.target, p.match, p.rev_p);
         }
     };
 
@@ -609,7 +631,7 @@ __global__ void __launch_bounds__(kThreads, AA ? GBSW_DUAL_MIN_BLOCKS
                     h[0].pad = REVERSE ? 0 : nstrips * W - h[0].ncols_run;
                     h[1].pad = REVERSE ? 0 : nstrips * W - h[1].ncols_run;
                     if constexpr (REVERSE) {
-                        sband[threadIdx.x] = unit_band(h[0], h[1]);
+                        sband[threadIdx.x] = make_int2(unit_band(h[0], h[1]), unit_low_band(h[0], h[1]));
                         tgt2 = pack16(h[0].target > 0 ? h[0].target + open : 0x7fff,
                                       h[1].target > 0 ? h[1].target + open : 0x7fff);
                     }
