@@ -56,7 +56,7 @@ __global__ void __launch_bounds__(256) probe_dual(int iters, int seed, int* sink
         pa[c] = 0xfd03fdfdu ^ (unsigned)(c * 0x01010101 * (seed & 1)) ^ base;
         pb[c] = 0x03fdfdfdu ^ (base << 1);
     }
-    const unsigned open2 = 0xfffafffau, ext2 = 0xffffffffu, neg2 = 0x80008000u;
+    const unsigned open2 = 0xfffafffau, ext2 = 0xffffffffu;
     unsigned e = threadIdx.x, mrow = 0, acc = 0;
     __syncthreads();
     long long t0 = clock64();
@@ -68,7 +68,7 @@ __global__ void __launch_bounds__(256) probe_dual(int iters, int seed, int* sink
         for (int c = 0; c < kDualCols; ++c) {
             const unsigned s2 = prmt_probe(pa[c], pb[c], sel);
             const unsigned fv = __viaddmax_s16x2_relu(f[c], ext2, ho[c]);
-            const unsigned u2 = __viaddmax_s16x2(diag, s2, neg2);
+            const unsigned u2 = __vadd2(diag, s2);
             const unsigned t = __viaddmax_s16x2(fv, open2, u2);
             const unsigned hov = __viaddmax_s16x2(e, open2, t);
             e = __viaddmax_s16x2_relu(e, ext2, t);

@@ -43,6 +43,14 @@
 //   Ho  = max(E + open, T)
 //   E'  = max(E + max(ext, open), T, 0)          (= max(E + ext, Ho, 0))
 // which is the int32 kernel's recurrence (see sw_pass.cuh) evaluated per half.
+// The plain packed add of T's second term runs beside the ALU pipe, which takes
+// a warp instruction every other cycle and bounds the kernel (measured: a
+// viaddmax alone 1.01 ns per warp and scheduler, with a packed add beside it
+// 1.01, with a second viaddmax, vimax3 or prmt 2.02): as a viaddmax with a third
+// operand that never wins it cost the 100,000-pair DNA forward 4.81 against
+// 4.62 ms, the mixed batch's long pairs 61.5 against 57.9 ms.  Turning more of the
+// recurrence into free adds (one vimax3 for the three-way H max, 4.5 ALU ops a
+// cell pair for 5.5) gained nothing on top: 4.61 ms.
 // Argmax rules and the transposed reverse pass are also the int32 kernel's,
 // band included (reverse_band, reverse_low_band): a unit's strips start and end
 // at the rows its wider band needs (unit_band, unit_low_band), and both halves
@@ -74,7 +82,6 @@ constexpr int kCD = GBSW_DUAL_DNA_COLS;
 // Long DNA pairs (the long bin's default plan): kDualWideLanes lanes x kCD columns.
 constexpr int kGDW = kDualWideLanes;
 static_assert(kGD * kCD == 64, "the schedule pairs DNA units by 64-column strips");
-constexpr unsigned kNeg2 = 0x80008000u;
 // Pipeline steps per loop iteration (even: boundary rows are copied in pairs;
 // at most 8: one code byte each in a 64-bit word).  Longer chunks cut the
 // per-iteration overhead but unroll the loop body further.  Measured on the
@@ -710,7 +717,7 @@ __global__ void __launch_bounds__(kThreads, AA ? GBSW_DUAL_MIN_BLOCKS
                             s2 = (c & 1) ? prmt2(pw.z, pw.w, sel) : prmt2(pw.x, pw.y, sel);
                         }
                         const unsigned fv = __viaddmax_s16x2_relu(f[c], ext2, ho[c]);  // F(i,j)
-                        const unsigned u2 = __viaddmax_s16x2(diag, s2, kNeg2);        // Ho_diag + s
+                        const unsigned u2 = __vadd2(diag, s2);                         // Ho_diag + s
                         const unsigned t = __viaddmax_s16x2(fv, open2, u2);           // max(F + open, .)
                         hov = __viaddmax_s16x2(e, open2, t);                          // Ho(i,j)
                         e = __viaddmax_s16x2_relu(e, gmax2, t);                       // E(i,j+1)
