@@ -13,6 +13,7 @@
 #include "pack.h"
 #include "schedule.h"
 #include "sw_kernels.h"
+#include "sw_strips.h"
 #include "results.h"
 #include "traceback.h"
 #include "tuning.h"
@@ -89,6 +90,11 @@ struct gbsw_context {
     DevBuf<int> d_hist;      // schedule: bucket counters / offsets, then the class ranges
     DevBuf<int> d_matrix;    // 25x25 (score - open)
     DevBuf<int> d_encoding;  // 91 entries
+    // strip-parallel passes: task list, edge buffers, read marks and the next unused tag
+    DevBuf<int2> d_tasks;
+    DevBuf<uint64_t> d_edges;
+    DevBuf<unsigned> d_freed;
+    unsigned strip_tag = 1;
     HostBuf<int> h_misc;
     // traceback
     DevBuf<uint32_t> d_tb_ops, d_tb_dir, d_tb_out;
@@ -104,6 +110,7 @@ struct gbsw_context {
     bool timed_host = false;
     gbsw_stats stats{};
     gbsw_tuning tuning = gbsw::builtin_tuning();  // per (kind, length bin, pair-count bucket) plans
+    bool tuning_builtin = true;                   // not replaced by the caller
 
     int fail(int code, const std::string& msg) {
         last_error = msg;
@@ -248,6 +255,47 @@ int dual_or_pass_occupancy(gbsw_context* ctx, bool protein, int score, bool rev,
     return GBSW_OK;
 }
 
+// Task room and edge buffers of the strip-parallel passes of one call.  A batch
+// whose strips could exceed kMaxStripTasks keeps the block-per-pair kernels
+// (those batches fill the GPU with pairs anyway).
+constexpr int64_t kMaxStripTasks = int64_t(1) << 24;
+constexpr int64_t kStripEdgeBytes = int64_t(1) << 29;
+
+// Reserves them for up to `tasks` tasks of one launch over sequences of up to
+// `rows` symbols: a buffer per task, but no more than four for every warp that
+// runs or than kStripEdgeBytes hold, and no fewer than those warps (fewer would
+// make tasks wait for buffers).
+int reserve_strips(gbsw_context* ctx, int64_t tasks, int rows, cudaStream_t stream, gbsw::StripParams* s) {
+    const int64_t stride = gbsw::strip_edge_stride(rows);
+    const int64_t resident = (int64_t)ctx->sms * 12;  // warps: three blocks of four an SM
+    const int64_t ring =
+        std::max<int64_t>(2, std::min({tasks, 4 * resident, std::max(resident, kStripEdgeBytes / (8 * stride))}));
+    const size_t edge_cap = ctx->d_edges.cap, freed_cap = ctx->d_freed.cap;
+    cudaError_t e = ctx->d_tasks.reserve((size_t)tasks);
+    if (e == cudaSuccess) e = ctx->d_edges.reserve((size_t)(ring * stride));
+    if (e == cudaSuccess) e = ctx->d_freed.reserve((size_t)tasks);
+    if (e != cudaSuccess) return ctx->fail(GBSW_ENOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+    // no word of a buffer may carry a tag that is still to come: new memory is
+    // cleared, and all of it when the tags start over (two launches a call and pass)
+    const bool fresh = ctx->d_edges.cap != edge_cap || ctx->d_freed.cap != freed_cap;
+    if (fresh || ctx->strip_tag > 0xffffffffu - (unsigned)(4 * tasks)) {
+        e = cudaMemsetAsync(ctx->d_edges.ptr, 0, sizeof(uint64_t) * ctx->d_edges.cap, stream);
+        if (e == cudaSuccess) e = cudaMemsetAsync(ctx->d_freed.ptr, 0, sizeof(unsigned) * ctx->d_freed.cap, stream);
+        if (e != cudaSuccess) return ctx->cuda_fail(e, "cudaMemsetAsync");
+        ctx->strip_tag = 1;
+    }
+    s->tasks = ctx->d_tasks.ptr;
+    s->ntasks = ctx->d_misc.ptr + 26;
+    s->on_sm = ctx->d_misc.ptr + 32;
+    s->max_tasks = (int)tasks;
+    s->freed = ctx->d_freed.ptr;
+    s->edges = ctx->d_edges.ptr;
+    s->edge_stride = (int)stride;
+    s->ring = (int)ring;
+    s->sms = ctx->sms;
+    return GBSW_OK;
+}
+
 // Enqueue the schedule and both passes for n pairs already on the device.
 // `tune` (gbsw_tune_device) forces every bin to one variant and times each
 // class launch with events; the result arrays are those of a normal call.
@@ -285,7 +333,7 @@ int run_passes(gbsw_context* ctx, const gbsw_scoring* sc, const uint8_t* ref, co
         for (int b = 0; b < gbsw::kBins; ++b)
             for (int k = 0; k < GBSW_COUNT_BUCKETS; ++k) use_table = use_table || table.variant[sc->kind][b][k].lanes > 0;
 
-    cudaError_t e = ctx->d_misc.reserve(32);
+    cudaError_t e = ctx->d_misc.reserve(32 + gbsw::kStripSmSlots);
     if (e == cudaSuccess) e = ctx->d_rerun.reserve((size_t)n + 2);
     if (e == cudaSuccess) e = ctx->d_cls.reserve((size_t)n);
     if (e == cudaSuccess) e = ctx->d_keys.reserve((size_t)n);
@@ -342,18 +390,32 @@ int run_passes(gbsw_context* ctx, const gbsw_scoring* sc, const uint8_t* ref, co
     // A caller that knows the bins' counts on the host (the serving loop) skips
     // the wait: the plan comes from its counts, a bin it counts empty is empty on
     // the device too, and the other ranges launch whatever they hold.
+    auto take_count = [&](int b, int64_t count) {
+        ctx->stats.bin_pairs[b] = count;
+        gbsw_variant v = table.variant[sc->kind][b][count_bucket(count)];
+        gbsw_variant rv = table.reverse[sc->kind][b][count_bucket(count)];
+        if (!use_table || count <= 0 || !variant_ok(protein, v, dual_ok)) return;
+        // Pairs of at most 512 symbols end soon even two to a group: 8,000 reads of
+        // 100-150 against 200-500 bp take 271 us forward so and 281 strip by strip, 4,000
+        // 258 and 177 (longer pairs: 8,000 of the throughput shape 875 and 604).
+        if (ctx->tuning_builtin && !protein && b == 0 && !v.dual && v.lanes == gbsw::kTeamLanes && count > 7000 &&
+            max_len <= 512)
+            v = rv = gbsw_variant{1, 16};
+        // A few long proteins among many short ones: one launch over both bins ends
+        // sooner once the short ones fill it (60,000 pairs, 6,215 of them long: 7.38
+        // against 7.68 ms for both passes; 34,000 pairs: 5.21 against 4.60).
+        if (ctx->tuning_builtin && protein && b == 1 && !v.dual && v.lanes == gbsw::kTeamLanes &&
+            plan.bin[0][0].dual && ctx->stats.bin_pairs[0] > 50000)
+            v = rv = plan.bin[0][0];
+        plan.bin[0][b] = plan.bin[1][b] = v;
+        if (variant_ok(protein, rv, dual_ok)) plan.bin[1][b] = rv;
+        plan.from_table[b] = true;
+    };
     if (host_bins && use_table && !tune) {
         for (int b = 0; b < gbsw::kBins; ++b) {
             const int64_t count = std::max<int64_t>(0, host_bins[b]);
             range_pairs[b ? gbsw::kRangeLong : gbsw::kRangeShort] = count;
-            ctx->stats.bin_pairs[b] = count;
-            const gbsw_variant& v = table.variant[sc->kind][b][count_bucket(count)];
-            if (count > 0 && variant_ok(protein, v, dual_ok)) {
-                plan.bin[0][b] = plan.bin[1][b] = v;
-                const gbsw_variant& rv = table.reverse[sc->kind][b][count_bucket(count)];
-                if (variant_ok(protein, rv, dual_ok)) plan.bin[1][b] = rv;
-                plan.from_table[b] = true;
-            }
+            take_count(b, count);
         }
     } else if (use_table || tune) {
         int* hr = ctx->h_misc.ptr + 32;
@@ -361,19 +423,34 @@ int run_passes(gbsw_context* ctx, const gbsw_scoring* sc, const uint8_t* ref, co
         if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
         if (e != cudaSuccess) return ctx->cuda_fail(e, "bin counts");
         for (int r = 0; r < gbsw::kRanges; ++r) range_pairs[r] = hr[2 * r + 1] - hr[2 * r];
-        for (int b = 0; b < gbsw::kBins; ++b) {
-            const int r = b ? gbsw::kRangeLong : gbsw::kRangeShort;
-            const int64_t count = hr[2 * r + 1] - hr[2 * r];
-            ctx->stats.bin_pairs[b] = count;
-            const gbsw_variant& v = table.variant[sc->kind][b][count_bucket(count)];
-            if (use_table && count > 0 && variant_ok(protein, v, dual_ok)) {
-                plan.bin[0][b] = plan.bin[1][b] = v;
-                const gbsw_variant& rv = table.reverse[sc->kind][b][count_bucket(count)];
-                if (variant_ok(protein, rv, dual_ok)) plan.bin[1][b] = rv;
-                plan.from_table[b] = true;
-            }
-        }
+        for (int b = 0; b < gbsw::kBins; ++b) take_count(b, range_pairs[b ? gbsw::kRangeLong : gbsw::kRangeShort]);
     }
+
+    // block-per-pair plans of the binned pairs run strip-parallel in int16x2
+    const int rows = (std::max(1, max_len) + 1) & ~1;  // even: 16-byte boundary copies stay in a group's buffer
+    auto strip_tasks = [&](int64_t pairs, int cols) {
+        return pairs * ((std::max(1, max_len) + gbsw::strip_width(cols) - 1) / gbsw::strip_width(cols));
+    };
+    // 8 columns a lane once the long pairs alone give every scheduler several strips
+    // of 4 (then the steps' fixed work counts, not the chain of one strip): 3,000 mixed
+    // pairs, 900 of them long, 1,435 against 1,502 us forward, 300 long reads 7.27
+    // against 8.17 ms; below that 4 win: 61 long reads 2.35 against 2.50 ms, 1,000
+    // mixed pairs 746 against 801 us.
+    const int64_t long_pairs = range_pairs[gbsw::kRangeLong] >= 0 ? range_pairs[gbsw::kRangeLong] : n;
+    const int strip_cols = gbsw::strip_columns(protein, strip_tasks(long_pairs, 4) >= 8192);
+    const int64_t strip_bound = strip_tasks(n, strip_cols);
+    const bool strips_fit = plan.binned && strip_bound <= kMaxStripTasks;
+    auto strips = [&](int rev, int b) {
+        return strips_fit && !plan.bin[rev][b].dual && plan.bin[rev][b].lanes == gbsw::kTeamLanes;
+    };
+    const bool any_strips[2] = {strips(0, 0) || strips(0, 1), strips(1, 0) || strips(1, 1)};
+    gbsw::StripParams strip_params{};
+    if (any_strips[0] || any_strips[1]) {
+        int rc = reserve_strips(ctx, strip_bound, rows, stream, &strip_params);
+        if (rc != GBSW_OK) return rc;
+    }
+    // their int16 overflows are long pairs: rerun block per pair
+    if (any_strips[0]) plan.int32_lanes = gbsw::kTeamLanes;
 
     // the bins share one launch over their whole class when their plans agree
     // (the tuner times them apart)
@@ -394,6 +471,19 @@ int run_passes(gbsw_context* ctx, const gbsw_scoring* sc, const uint8_t* ref, co
             for (int b = 0; b < gbsw::kBins; ++b) {
                 const int cls = b ? gbsw::kRangeLong : gbsw::kRangeShort;
                 const gbsw_variant& v = plan.bin[rev][b];
+                if (strips(rev, b)) {
+                    // a warp per task, spread over the SMs before they stack up
+                    int per_sm = ctx->opts.blocks_per_sm;
+                    if (per_sm <= 0) {
+                        e = gbsw::strips_occupancy(rev != 0, protein, strip_cols, &per_sm);
+                        if (e != cudaSuccess) return ctx->cuda_fail(e, "occupancy");
+                    }
+                    const int64_t want = (strip_bound + 3) / 4;
+                    per_sm = std::min(per_sm, 3);
+                    grid[rev][cls] = (int)std::min<int64_t>((int64_t)ctx->sms * std::max(1, per_sm),
+                                                            std::max<int64_t>(ctx->sms, want));
+                    continue;
+                }
                 int rc = dual_or_pass_occupancy(ctx, protein, score_mode(sc, 0, dna_profile_ok, aa_profile_ok),
                                                 rev != 0, dpx, v, &grid[rev][cls]);
                 if (rc != GBSW_OK) return rc;
@@ -403,7 +493,6 @@ int run_passes(gbsw_context* ctx, const gbsw_scoring* sc, const uint8_t* ref, co
             grid[rev][gbsw::kClassBinned] = grid[rev][gbsw::kRangeShort];
         }
     }
-    const int rows = (std::max(1, max_len) + 1) & ~1;  // even: 16-byte boundary copies stay in a group's buffer
     e = ctx->d_scratch.reserve((size_t)groups * (size_t)rows);
     if (e != cudaSuccess) return ctx->fail(GBSW_ENOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
 
@@ -447,17 +536,20 @@ int run_passes(gbsw_context* ctx, const gbsw_scoring* sc, const uint8_t* ref, co
     // takes no pair whose score may exceed int16 (reverse_keys sends those to
     // class 0)
     const bool any_dual = plan.any_dual(0) || plan.any_dual(1);
+    const bool any_int16 = any_dual || any_strips[0] || any_strips[1];
     // A range known to be empty needs no launch.  A pair keeps its forward
     // range in the reverse pass, except pairs with no score (to the idle class)
     // and dual-pair pairs rerun in int32 (to class 0), so class 0's reverse
     // launch stays whenever a dual launch could have queued reruns.
     auto empty = [&](int rev, int range) {
         if (range_pairs[range] != 0) return false;
-        return !(rev && range == 0 && any_dual);
+        return !(rev && range == 0 && any_int16);
     };
     for (int rev = 0; rev < 2; ++rev) {
         if (rev) {
-            sp.rev_dual_bins = plan.binned ? (plan.bin[1][0].dual ? 1 : 0) | (plan.bin[1][1].dual ? 2 : 0) : 0;
+            sp.rev_dual_bins = plan.binned ? (plan.bin[1][0].dual || strips(1, 0) ? 1 : 0) |
+                                                 (plan.bin[1][1].dual || strips(1, 1) ? 2 : 0)
+                                           : 0;
             e = gbsw::build_schedule(sp, true, ctx->sms, stream);
             if (e != cudaSuccess) return ctx->cuda_fail(e, "schedule");
             launches += 3;
@@ -477,6 +569,12 @@ int run_passes(gbsw_context* ctx, const gbsw_scoring* sc, const uint8_t* ref, co
                 p.cls = cls;
                 p.queue = queue(cls);
                 e = timed(rev, cls, [&] {
+                    if (strips(rev, b)) {
+                        strip_params.tag_base = ctx->strip_tag;
+                        ctx->strip_tag += (unsigned)strip_bound;
+                        ++launches;
+                        return gbsw::launch_strips(rev != 0, protein, strip_cols, p, strip_params, grid[rev][cls], stream);
+                    }
                     return v.dual ? gbsw::launch_pass_dual(rev != 0, protein, v.lanes, p, grid[rev][cls], stream)
                                   : gbsw::launch_pass(score_mode(sc, 0, dna_profile_ok, aa_profile_ok), rev != 0, dpx,
                                                       v.lanes, p, grid[rev][cls], stream);
@@ -494,7 +592,7 @@ int run_passes(gbsw_context* ctx, const gbsw_scoring* sc, const uint8_t* ref, co
             if (e != cudaSuccess) return ctx->cuda_fail(e, rev ? "reverse pass launch" : "forward pass launch");
             ++launches;
         }
-        if (plan.any_dual(0) && !rev) {
+        if ((plan.any_dual(0) || any_strips[0]) && !rev) {
             // the dual-pair pairs that may have overflowed int16, in the int32
             // class-0 kernel: its work list is the rerun list the dual launches
             // above filled (class range [rerun[0], rerun[1]) = [0, count))
@@ -513,7 +611,7 @@ int run_passes(gbsw_context* ctx, const gbsw_scoring* sc, const uint8_t* ref, co
     ctx->stats.launches = launches;
     ctx->stats.lane_group = plan.binned ? plan.bin[0][0].lanes : plan.int32_lanes;
     ctx->stats.dual = any_dual ? 1 : 0;
-    ctx->stats.reruns = plan.any_dual(0) ? -1 : 0;  // read back on demand (gbsw_last_stats)
+    ctx->stats.reruns = plan.any_dual(0) || any_strips[0] ? -1 : 0;  // read back on demand (gbsw_last_stats)
     for (int b = 0; b < gbsw::kBins; ++b) {
         ctx->stats.bin_dual[b] = plan.binned ? plan.bin[0][b].dual : 0;
         ctx->stats.bin_lanes[b] = plan.binned ? plan.bin[0][b].lanes : plan.int32_lanes;
@@ -1047,6 +1145,9 @@ void gbsw_destroy(gbsw_context* ctx) {
     ctx->d_scratch.release();
     ctx->d_misc.release();
     ctx->d_rerun.release();
+    ctx->d_tasks.release();
+    ctx->d_edges.release();
+    ctx->d_freed.release();
     ctx->d_matrix.release();
     ctx->d_encoding.release();
     ctx->d_cls.release();
@@ -1205,6 +1306,7 @@ int gbsw_set_tuning(gbsw_context* ctx, const gbsw_tuning* tuning) {
                         return ctx->fail(GBSW_EINVAL, "tuning: no kernel variant with these lanes");
                 }
     ctx->tuning = *tuning;
+    ctx->tuning_builtin = false;
     return GBSW_OK;
 }
 
@@ -1272,6 +1374,7 @@ int gbsw_tune_device(gbsw_context* ctx, const gbsw_scoring* scoring, const uint8
     }
     report->ncandidates = nc;
     if (nc == 0) return ctx->fail(GBSW_EINVAL, "no kernel variant applies to this scoring");
+    ctx->tuning_builtin = false;
     // the bins' pair counts, as the forward schedule of the last run found them
     for (int b = 0; b < GBSW_BINS; ++b) {
         report->pairs[b] = ctx->stats.bin_pairs[b];
