@@ -26,9 +26,10 @@ struct StripParams {
 };
 
 // Entries of an edge buffer for sequences of up to `rows` symbols: the rows, 128
-// before them and 8 after (the pipeline's fill and the last chunk's rest), and
-// the two words of the best.
-inline int strip_edge_stride(int rows) { return (rows + 128 + 8 + 2 + 1) & ~1; }
+// before them and 16 after (the pipeline's fill and the rest of the last chunk: up
+// to 7 steps of two rows past the step of the last row, 15 with an odd last row),
+// and the two words of the best.
+inline int strip_edge_stride(int rows) { return (rows + 128 + 16 + 2 + 1) & ~1; }
 // Columns of a strip with `columns` (4 or 8) columns a lane.
 __host__ __device__ constexpr int strip_width(int columns) { return 64 * columns; }
 // Columns a lane holds: 8 where there is a kernel for them and `wide` is asked for.
