@@ -102,6 +102,7 @@ struct gbsw_context {
     DevBuf<int64_t> d_tb_off;    // slot, direction, boundary and output offsets: 4n + 1
     DevBuf<int32_t> d_tb_count;  // operations and path score per pair: 2n
     HostBuf<int64_t> h_tb_off;
+    HostBuf<int2> h_tb_tasks;    // int16 kernel: strip tasks of all launches
     HostBuf<int32_t> h_tb_count;
     HostBuf<uint32_t> h_tb_ops;
 
@@ -261,11 +262,12 @@ int dual_or_pass_occupancy(gbsw_context* ctx, bool protein, int score, bool rev,
 constexpr int64_t kMaxStripTasks = int64_t(1) << 24;
 constexpr int64_t kStripEdgeBytes = int64_t(1) << 29;
 
-// Reserves them for up to `tasks` tasks of one launch over sequences of up to
-// `rows` symbols: a buffer per task, but no more than four for every warp that
+// Reserves them for up to `tasks` tasks of one launch and `tags` of all the call's,
+// over sequences of up to `rows` symbols: a buffer per task, but no more than four for every warp that
 // runs or than kStripEdgeBytes hold, and no fewer than those warps (fewer would
 // make tasks wait for buffers).
-int reserve_strips(gbsw_context* ctx, int64_t tasks, int rows, cudaStream_t stream, gbsw::StripParams* s) {
+int reserve_strips(gbsw_context* ctx, int64_t tasks, int64_t tags, int rows, cudaStream_t stream,
+                   gbsw::StripParams* s) {
     const int64_t stride = gbsw::strip_edge_stride(rows);
     const int64_t resident = (int64_t)ctx->sms * 12;  // warps: three blocks of four an SM
     const int64_t ring =
@@ -276,9 +278,9 @@ int reserve_strips(gbsw_context* ctx, int64_t tasks, int rows, cudaStream_t stre
     if (e == cudaSuccess) e = ctx->d_freed.reserve((size_t)tasks);
     if (e != cudaSuccess) return ctx->fail(GBSW_ENOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
     // no word of a buffer may carry a tag that is still to come: new memory is
-    // cleared, and all of it when the tags start over (two launches a call and pass)
+    // cleared, and all of it when the tags start over
     const bool fresh = ctx->d_edges.cap != edge_cap || ctx->d_freed.cap != freed_cap;
-    if (fresh || ctx->strip_tag > 0xffffffffu - (unsigned)(4 * tasks)) {
+    if (fresh || (int64_t)ctx->strip_tag + tags > (int64_t)0xffffffff) {
         e = cudaMemsetAsync(ctx->d_edges.ptr, 0, sizeof(uint64_t) * ctx->d_edges.cap, stream);
         if (e == cudaSuccess) e = cudaMemsetAsync(ctx->d_freed.ptr, 0, sizeof(unsigned) * ctx->d_freed.cap, stream);
         if (e != cudaSuccess) return ctx->cuda_fail(e, "cudaMemsetAsync");
@@ -446,7 +448,7 @@ int run_passes(gbsw_context* ctx, const gbsw_scoring* sc, const uint8_t* ref, co
     const bool any_strips[2] = {strips(0, 0) || strips(0, 1), strips(1, 0) || strips(1, 1)};
     gbsw::StripParams strip_params{};
     if (any_strips[0] || any_strips[1]) {
-        int rc = reserve_strips(ctx, strip_bound, rows, stream, &strip_params);
+        int rc = reserve_strips(ctx, strip_bound, 4 * strip_bound, rows, stream, &strip_params);
         if (rc != GBSW_OK) return rc;
     }
     // their int16 overflows are long pairs: rerun block per pair
@@ -688,9 +690,12 @@ int decode_device_error(gbsw_context* ctx, int flags) {
     return GBSW_OK;
 }
 
-// Device bytes of direction words plus strip boundaries one traceback launch
-// may hold; larger batches run in several launches.
+// Device bytes of direction words plus strip boundaries one traceback launch may
+// hold; larger batches run in several launches.  kTraceBudget always, kTraceBudgetFree
+// while at most half of the free memory goes to it: each launch ends with its longest
+// paths' walks (100,000 DNA pairs in three launches 1.28 ms of walks, in one 0.57).
 constexpr int64_t kTraceBudget = int64_t(1) << 30;
+constexpr int64_t kTraceBudgetFree = int64_t(5) << 30;
 
 int traceback_host(gbsw_context* ctx, const gbsw_scoring* sc, const char* ref, const int64_t* ref_off,
                    const char* query, const int64_t* query_off, int64_t n, const int32_t* top_scores,
@@ -714,6 +719,22 @@ int traceback_host(gbsw_context* ctx, const gbsw_scoring* sc, const char* ref, c
 
     cudaError_t e = cudaSetDevice(ctx->device);
     if (e != cudaSuccess) return ctx->cuda_fail(e, "cudaSetDevice");
+    // The int16x2 kernel (trace_strips.cu) takes the pairs whose values fit it, the
+    // int32 kernel (traceback.cu) the others.
+    const bool protein = sc->kind == GBSW_PROTEIN;
+    bool int8_scores = protein || (fits_int8(sc->match) && fits_int8(sc->mismatch));
+    int best = protein ? 0 : (int)sc->match;
+    if (protein)
+        for (int k = 0; k < 576; ++k) {
+            int8_scores = int8_scores && fits_int8(sc->matrix[k]);
+            best = std::max(best, (int)sc->matrix[k]);
+        }
+    const bool scores16 =
+        gbsw::trace16_scores_ok(int8_scores, sc->match, sc->mismatch, protein, sc->gap_open, sc->gap_extend);
+    const gbsw::Trace16Limits lim16 = gbsw::trace16_limits(best, sc->gap_open, sc->gap_extend);
+    auto fits16 = [&](int m, int kk, int score) {
+        return scores16 && gbsw::trace16_pair_ok(lim16, m, kk, score, sc->gap_open, sc->gap_extend);
+    };
     // per pair: operation slot (m + k), direction words and boundary entries of
     // its launch; launches cut where the budget fills
     e = ctx->h_tb_off.reserve((size_t)5 * n + 1);
@@ -721,9 +742,10 @@ int traceback_host(gbsw_context* ctx, const gbsw_scoring* sc, const char* ref, c
     int64_t* slot = ctx->h_tb_off.ptr;       // n + 1
     int64_t* dir_off = slot + n + 1;         // n
     int64_t* bnd_off = dir_off + n;          // n
-    int64_t* order = slot + 4 * n + 1;       // n: each launch's pairs by descending cost
+    int64_t* order = slot + 4 * n + 1;       // n: each launch's pairs by descending cost, int16 ones first
     std::vector<int64_t> cuts{0};
-    int64_t dir_max = 1, bnd_max = 1, dir_run = 0, bnd_run = 0;
+    int64_t dir_max = 1, bnd_max = 1, dir_run = 0, bnd_run = 0, total_tasks = 0, total_bytes = 0;
+    int rows16 = 1;  // largest row count (k + 1) of an int16 pair
     slot[0] = 0;
     for (int64_t k = 0; k < n; ++k) {
         int64_t cap = 0, dw = 0, bw = 0;
@@ -734,10 +756,32 @@ int traceback_host(gbsw_context* ctx, const gbsw_scoring* sc, const char* ref, c
                 return ctx->fail(GBSW_EINVAL, "traceback: begins/ends out of range for pair " + std::to_string(k));
             const int m = ref_end[k] - ref_begin[k], kk = query_end[k] - query_begin[k];
             cap = (int64_t)m + kk;
-            dw = gbsw::trace_dir_words(m, kk);
-            bw = (int64_t)kk + 1;
+            if (fits16(m, kk, top_scores[k])) {
+                dw = gbsw::trace16_dir_words(m, kk);
+                total_tasks += (m + gbsw::kTrace16Width - 1) / gbsw::kTrace16Width;
+                rows16 = std::max(rows16, kk + 1);
+            } else {
+                dw = gbsw::trace_dir_words(m, kk);
+                bw = (int64_t)kk + 1;
+            }
         }
-        if (k > cuts.back() && (dir_run + dw) * 4 + (bnd_run + bw) * 8 > kTraceBudget) {
+        dir_off[k] = dw = (dw + 7) & ~(int64_t)7;  // whole sectors
+        bnd_off[k] = bw;
+        total_bytes += dw * 4 + bw * 8;
+        slot[k + 1] = slot[k] + cap;
+    }
+    int64_t budget = kTraceBudget;
+    if (total_bytes > budget) {
+        const int64_t want = std::min(kTraceBudgetFree, total_bytes), held = (int64_t)ctx->d_tb_dir.cap * 4;
+        size_t free_bytes = 0, all_bytes = 0;
+        if (held >= want)
+            budget = want;
+        else if (cudaMemGetInfo(&free_bytes, &all_bytes) == cudaSuccess)
+            budget = std::max(budget, std::min(want, held + (int64_t)(free_bytes / 2)));
+    }
+    for (int64_t k = 0; k < n; ++k) {
+        const int64_t dw = dir_off[k], bw = bnd_off[k];
+        if (k > cuts.back() && (dir_run + dw) * 4 + (bnd_run + bw) * 8 > budget) {
             cuts.push_back(k);
             dir_run = bnd_run = 0;
         }
@@ -747,40 +791,59 @@ int traceback_host(gbsw_context* ctx, const gbsw_scoring* sc, const char* ref, c
         bnd_run += bw;
         dir_max = std::max(dir_max, dir_run);
         bnd_max = std::max(bnd_max, bnd_run);
-        slot[k + 1] = slot[k] + cap;
     }
     cuts.push_back(n);
-    // Each launch's pairs by descending row steps (strips x (rows + fill)), so
-    // that the pairs a warp's groups run together end close together: a
-    // counting sort over 8 buckets per doubling of the cost (the exponent and
-    // the next three bits of the integer cost).
+    // Each launch's pairs by descending row steps (int16: strips x (row pairs + fill),
+    // int32: strips x (rows + fill)), so that the pairs a warp's groups or walks run
+    // together end close together: a counting sort over 8 buckets per doubling of
+    // the cost (the exponent and the next three bits of the integer cost).
+    const size_t launches = cuts.size() - 1;
+    std::vector<int64_t> count16(launches), first_task(launches + 1);  // per launch: int16 pairs, their tasks
+    int64_t max_tasks = 0;
+    e = ctx->h_tb_tasks.reserve((size_t)std::max<int64_t>(total_tasks, 1));
+    if (e != cudaSuccess) return ctx->fail(GBSW_ENOMEM, "cudaMallocHost");
     {
         constexpr int kCostBuckets = 8 * 64;
         std::vector<uint16_t> bucket((size_t)n);
         for (int64_t k = 0; k < n; ++k) {
-            int b = 0;
+            int b = 0, wide = 0;
             if (top_scores[k] > 0) {
                 const int m = ref_end[k] - ref_begin[k], kk = query_end[k] - query_begin[k];
-                const uint64_t cost = (uint64_t)((m + gbsw::kTraceCols - 1) / gbsw::kTraceCols) *
-                                      (uint64_t)(kk + gbsw::kTraceLanes - 1);
+                wide = fits16(m, kk, top_scores[k]) ? 0 : 1;
+                const uint64_t cost = wide ? (uint64_t)((m + gbsw::kTraceCols - 1) / gbsw::kTraceCols) *
+                                                 (uint64_t)(kk + gbsw::kTraceLanes - 1)
+                                           : (uint64_t)((m + gbsw::kTrace16Width - 1) / gbsw::kTrace16Width) *
+                                                 (uint64_t)(kk / 2 + 64);
                 const int e = 63 - __builtin_clzll(cost | 1);
                 const int frac = e >= 3 ? (int)((cost >> (e - 3)) & 7) : (int)((cost << (3 - e)) & 7);
                 b = std::min(kCostBuckets - 1, 1 + 8 * e + frac);
             }
-            bucket[(size_t)k] = (uint16_t)(kCostBuckets - 1 - b);  // descending cost first
+            bucket[(size_t)k] = (uint16_t)(wide * kCostBuckets + kCostBuckets - 1 - b);  // descending cost first
         }
-        std::vector<int64_t> count(kCostBuckets);
-        for (size_t c = 0; c + 1 < cuts.size(); ++c) {
+        std::vector<int64_t> count(2 * kCostBuckets);
+        int2* tasks = ctx->h_tb_tasks.ptr;
+        int64_t nt = 0;
+        for (size_t c = 0; c < launches; ++c) {
             std::fill(count.begin(), count.end(), 0);
             for (int64_t k = cuts[c]; k < cuts[c + 1]; ++k) ++count[bucket[(size_t)k]];
             int64_t at = cuts[c];
-            for (int b = 0; b < kCostBuckets; ++b) {
+            for (int b = 0; b < 2 * kCostBuckets; ++b) {
+                if (b == kCostBuckets) count16[c] = at - cuts[c];
                 const int64_t here = count[b];
                 count[b] = at;
                 at += here;
             }
             for (int64_t k = cuts[c]; k < cuts[c + 1]; ++k) order[count[bucket[(size_t)k]]++] = k;
+            first_task[c] = nt;
+            for (int64_t x = cuts[c]; x < cuts[c] + count16[c]; ++x) {
+                const int64_t k = order[x];
+                if (top_scores[k] <= 0) continue;
+                const int strips = (ref_end[k] - ref_begin[k] + gbsw::kTrace16Width - 1) / gbsw::kTrace16Width;
+                for (int t = 0; t < strips; ++t) tasks[nt++] = make_int2((int)k, t | (strips << 16));
+            }
+            max_tasks = std::max(max_tasks, nt - first_task[c]);
         }
+        first_task[launches] = nt;
     }
     const int64_t ra = ref_off[n], qa = query_off[n];
     cudaStream_t stream = ctx->stream;
@@ -795,8 +858,14 @@ int traceback_host(gbsw_context* ctx, const gbsw_scoring* sc, const char* ref, c
     if (e == cudaSuccess) e = ctx->d_tb_bnd.reserve((size_t)bnd_max);
     if (e == cudaSuccess) e = ctx->d_tb_off.reserve((size_t)5 * n + 1);
     if (e == cudaSuccess) e = ctx->d_tb_count.reserve((size_t)2 * n);
-    if (e == cudaSuccess) e = ctx->d_misc.reserve(8);
+    if (e == cudaSuccess) e = ctx->d_misc.reserve(32 + gbsw::kStripSmSlots);
+    if (e == cudaSuccess) e = ctx->d_tasks.reserve((size_t)std::max<int64_t>(total_tasks, 1));
     if (e != cudaSuccess) return ctx->fail(GBSW_ENOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+    gbsw::StripParams strip_params{};
+    if (max_tasks > 0) {
+        rc = reserve_strips(ctx, max_tasks, total_tasks, rows16, stream, &strip_params);
+        if (rc != GBSW_OK) return rc;
+    }
     e = ctx->h_tb_count.reserve((size_t)n);
     if (e == cudaSuccess) e = ctx->h_misc.reserve(16);
     if (e != cudaSuccess) return ctx->fail(GBSW_ENOMEM, "cudaMallocHost");
@@ -809,7 +878,7 @@ int traceback_host(gbsw_context* ctx, const gbsw_scoring* sc, const char* ref, c
     // phases for gbsw_last_stats: copies in (h2d_ms), the traceback kernels
     // (forward_ms), the operations back (d2h_ms)
     ctx->stats = gbsw_stats{};
-    ctx->stats.launches = (int32_t)cuts.size() + 1;
+    ctx->stats.launches = 1;  // the gather of the operations, and the kernels below
     cudaEventRecord(ctx->ev[EV_START], stream);
     if (ra > 0) e = cudaMemcpyAsync(ctx->d_ref.ptr, ref, (size_t)ra, cudaMemcpyHostToDevice, stream);
     if (e == cudaSuccess && qa > 0)
@@ -828,6 +897,9 @@ int traceback_host(gbsw_context* ctx, const gbsw_scoring* sc, const char* ref, c
         e = cudaMemcpyAsync(d_off, slot, sizeof(int64_t) * (size_t)(3 * n + 1), cudaMemcpyHostToDevice, stream);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(d_off + 4 * n + 1, order, sizeof(int64_t) * (size_t)n, cudaMemcpyHostToDevice, stream);
+    if (e == cudaSuccess && total_tasks > 0)
+        e = cudaMemcpyAsync(ctx->d_tasks.ptr, ctx->h_tb_tasks.ptr, sizeof(int2) * (size_t)total_tasks,
+                            cudaMemcpyHostToDevice, stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(ctx->d_misc.ptr, 0, sizeof(int) * 8, stream);
     if (e != cudaSuccess) return ctx->cuda_fail(e, "traceback copies");
     cudaEventRecord(ctx->ev[EV_H2D], stream);
@@ -856,13 +928,38 @@ int traceback_host(gbsw_context* ctx, const gbsw_scoring* sc, const char* ref, c
     tp.nops = ctx->d_tb_count.ptr;
     tp.path_score = ctx->d_tb_count.ptr + n;
     tp.error = ctx->d_misc.ptr + 3;
-    for (size_t c = 0; c + 1 < cuts.size(); ++c) {
+    tp.queue = ctx->d_misc.ptr + 8;
+    tp.neg = lim16.neg;
+    tp.top = lim16.top;
+    int trace16_blocks = 0;
+    if (max_tasks > 0) {
+        e = gbsw::trace16_occupancy(protein, &trace16_blocks);
+        if (e != cudaSuccess) return ctx->cuda_fail(e, "occupancy");
+    }
+    for (size_t c = 0; c < launches; ++c) {
+        const int64_t ntasks = first_task[c + 1] - first_task[c];
         tp.first = cuts[c];
-        tp.count = cuts[c + 1] - cuts[c];
         // offsets are per launch; the kernel indexes them by pair within the launch
         tp.dir_off = d_off + (n + 1) + cuts[c];
         tp.bnd_off = d_off + (2 * n + 1) + cuts[c];
         tp.order = d_off + (4 * n + 1) + cuts[c];
+        tp.count = count16[c];
+        if (ntasks > 0) {
+            // the queue and the counters of blocks by SM
+            e = cudaMemsetAsync(tp.queue, 0, sizeof(int) * (24 + gbsw::kStripSmSlots), stream);
+            if (e != cudaSuccess) return ctx->cuda_fail(e, "cudaMemsetAsync");
+            strip_params.tasks = ctx->d_tasks.ptr + first_task[c];
+            strip_params.tag_base = ctx->strip_tag;
+            ctx->strip_tag += (unsigned)ntasks;
+        }
+        const int64_t blocks = std::min<int64_t>((int64_t)ctx->sms * std::max(1, trace16_blocks),
+                                                 std::max<int64_t>(ctx->sms, (ntasks + 3) / 4));
+        e = gbsw::launch_trace16(tp, strip_params, (int)ntasks, (int)blocks, stream);
+        if (e != cudaSuccess) return ctx->cuda_fail(e, "traceback launch");
+        ctx->stats.launches += (ntasks > 0) + (tp.count > 0);
+        tp.order += count16[c];
+        tp.count = cuts[c + 1] - cuts[c] - count16[c];
+        ctx->stats.launches += tp.count > 0;
         e = gbsw::launch_trace(tp, stream);
         if (e != cudaSuccess) return ctx->cuda_fail(e, "traceback launch");
     }
@@ -1162,6 +1259,7 @@ void gbsw_destroy(gbsw_context* ctx) {
     ctx->d_tb_off.release();
     ctx->d_tb_count.release();
     ctx->h_tb_off.release();
+    ctx->h_tb_tasks.release();
     ctx->h_tb_count.release();
     ctx->h_tb_ops.release();
     for (int k = 0; k < EV_COUNT; ++k)

@@ -46,6 +46,7 @@
 #include <algorithm>
 
 #include "sw_common.cuh"
+#include "strip_device.cuh"
 #include "sw_device.cuh"
 #include "sw_strips.h"
 
@@ -55,35 +56,11 @@ namespace {
 constexpr int kStripSteps = 8;                // steps of a chunk
 constexpr int kStripRows = 2 * kStripSteps;   // their rows, fetched together
 constexpr int kHalfLag = 64;                  // rows the high halves run behind the low ones
-// Polls of a wait before it gives up (each sleeps about 40 ns, so over a second).
-constexpr int kStripSpin = 1 << 25;
 // Entries of an edge buffer before row 1: the rows the last lane passes while
 // the pipeline fills (even: a step's two rows are stored together).
 constexpr int kEdgeFront = 128;
-constexpr unsigned kFull = 0xffffffffu;
 constexpr unsigned kPadCode = 4;  // DNA row code outside the pair
 constexpr unsigned kSelTableLo = 0xB3A29180u, kSelTableHi = 0x88u;  // selector byte of a row code (sw_dual.cu)
-
-__device__ __forceinline__ unsigned prmt(unsigned a, unsigned b, unsigned sel) {
-    unsigned r;
-    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(sel));
-    return r;
-}
-__device__ __forceinline__ int lo16(unsigned x) { return (int)(short)(x & 0xffffu); }
-__device__ __forceinline__ int hi16(unsigned x) { return (int)(short)(x >> 16); }
-__device__ __forceinline__ unsigned pack16(int lo, int hi) {
-    return (unsigned)(lo & 0xffff) | ((unsigned)hi << 16);
-}
-__device__ __forceinline__ uint64_t load_word(const uint64_t* p) {
-    uint64_t v;
-    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void store_words(uint64_t* p, unsigned tag, unsigned v, unsigned w) {
-    asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(((uint64_t)tag << 32) | v),
-                 "l"(((uint64_t)tag << 32) | w)
-                 : "memory");
-}
 
 // One pair as a pass sees it: rows stream, columns are held in registers.
 struct PairView {
@@ -212,41 +189,15 @@ __global__ void __launch_bounds__(kThreads, 4) sw_strips(PassParams p, StripPara
     const unsigned gmax2 = pack16(max(open, ext), max(open, ext));
     const unsigned zero_edge = (unsigned)open & 0xffffu;  // H = 0, E = 0
     const int ntasks = min(*s.ntasks, s.max_tasks);
-    // Warps that share a scheduler slow the chain of the longest pair, so few tasks
-    // keep one or two blocks to an SM and the others leave (measured by tasks per
-    // scheduler: 500 proteins, 1.2 of them, forward 178 us at one block, 225 at two,
-    // 262 at four; 1,000 mixed DNA pairs, 5 of them, 893, 762, 752 at three).  A
-    // block takes its warps' first tasks together, a warp its next ones alone.
     __shared__ int s_first;
-    if (threadIdx.x == 0) {
-        const int schedulers = s.sms * (kThreads / 32);
-        const int per_sm = ntasks <= 2 * schedulers ? 1 : (ntasks <= 4 * schedulers ? 2 : 64);
-        unsigned sm;
-        asm volatile("mov.u32 %0, %%smid;" : "=r"(sm));
-        s_first = atomicAdd(s.on_sm + sm % kStripSmSlots, 1) < per_sm ? atomicAdd(p.queue, kThreads / 32) : ntasks;
-    }
+    if (threadIdx.x == 0) s_first = strip_first_task(s, p.queue, ntasks);
     __syncthreads();
     int task = s_first + warp;
 
     unsigned char* const prof = sdyn + (REVERSE ? 0 : strip_row_bytes(C)) + (size_t)threadIdx.x * C;
 
-    // Polls until every lane that `needs` has `tag` on its word at `at`; false if
-    // the wait ran out (or another one did).
     auto wait_words = [&](bool needs, const uint64_t* at, unsigned tag, uint64_t& v) -> bool {
-        bool ready = !needs || (unsigned)(v >> 32) == tag;
-        for (int it = 0; !__all_sync(kFull, ready); ++it) {
-            const bool stop = it == kStripSpin || ((it & 1023) == 1023 && (*(volatile int*)p.error & kErrTeam));
-            if (__any_sync(kFull, stop)) {
-                if (lane == 0) atomicOr(p.error, kErrTeam);
-                return false;
-            }
-            __nanosleep(40);
-            if (!ready) {
-                v = load_word(at);
-                ready = (unsigned)(v >> 32) == tag;
-            }
-        }
-        return true;
+        return strip_wait(p.error, needs, at, tag, v);
     };
 
     // the next task (every warp runs its tasks in increasing order)
@@ -290,24 +241,7 @@ __global__ void __launch_bounds__(kThreads, 4) sw_strips(PassParams p, StripPara
         const uint64_t* const e_in = s.edges + (size_t)((task + s.ring - 1) % s.ring) * s.edge_stride;
         const bool writes = lane == 31;
         uint64_t* e_step = e_out + (kEdgeFront + 2 * (t - 63));
-        // the reader of this buffer's previous task must be done with it
-        if (!last && task >= s.ring) {
-            const int2 before = s.tasks[task - s.ring];
-            if ((before.y & 0xffff) + 1 < (int)((unsigned)before.y >> 16)) {
-                const volatile unsigned* f = s.freed + (task - s.ring);
-                const unsigned want = s.tag_base + (unsigned)(task - s.ring);
-                bool ok = false;
-                for (int it = 0; it < kStripSpin && !ok; ++it) {
-                    ok = *f == want;
-                    if (!ok && (it & 1023) == 1023 && (*(volatile int*)p.error & kErrTeam)) break;
-                    if (!ok) __nanosleep(40);
-                }
-                if (!__all_sync(kFull, ok)) {
-                    if (lane == 0) atomicOr(p.error, kErrTeam);
-                    break;
-                }
-            }
-        }
+        if (!last && !strip_buffer_free(p.error, s, task)) break;
 
         // ---- column profiles ----
         unsigned pa[AA ? 1 : C], pb[AA ? 1 : C];
@@ -594,7 +528,7 @@ __global__ void __launch_bounds__(kThreads, 4) sw_strips(PassParams p, StripPara
             const uint64_t left = ((uint64_t)__shfl_sync(kFull, (unsigned)v, 1) << 32) |
                                   __shfl_sync(kFull, (unsigned)v, 0);
             best = REVERSE ? (left < best ? left : best) : (left > best ? left : best);
-            if (lane == 0) *(volatile unsigned*)(s.freed + (task - 1)) = tag - 1;
+            if (lane == 0) strip_buffer_read(s, task - 1);
         }
         if (!last) {
             if (lane == 0)

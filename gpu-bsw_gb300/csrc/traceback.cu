@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(kTraceThreads) trace_pairs(TraceParams p) {
     final_h = __shfl_sync(gmask, final_h, mc / C, TG);
     if (g != 0) return;
     p.path_score[pid] = final_h;
-    uint32_t* out = p.ops + p.slot_off[pid];
+    uint32_t* out = p.ops + p.slot_off[pid + 1];  // written backwards: path order
     if (final_h != score) {
         atomicOr(p.error, kErrTrace);
         p.nops[pid] = 0;
@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(kTraceThreads) trace_pairs(TraceParams p) {
         if ((run & 15u) == op) {
             run += 16u;
         } else {
-            if (run) out[n++] = run;
+            if (run) *--out = run, ++n;
             run = 16u | op;
         }
     };
@@ -241,12 +241,7 @@ __global__ void __launch_bounds__(kTraceThreads) trace_pairs(TraceParams p) {
             --i;
         }
     }
-    if (run) out[n++] = run;
-    for (int x = 0, y = n - 1; x < y; ++x, --y) {
-        const uint32_t tmp = out[x];
-        out[x] = out[y];
-        out[y] = tmp;
-    }
+    if (run) *--out = run, ++n;
     p.nops[pid] = n;
 }
 
@@ -255,7 +250,7 @@ __global__ void gather_ops(const uint32_t* ops, const int64_t* slot_off, const i
     const int lane = threadIdx.x & 31;
     const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     for (int64_t k = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < n; k += warps) {
-        const uint32_t* src = ops + slot_off[k];
+        const uint32_t* src = ops + slot_off[k + 1] - nops[k];
         uint32_t* dst = out + out_off[k];
         for (int x = lane; x < nops[k]; x += 32) dst[x] = src[x];
     }

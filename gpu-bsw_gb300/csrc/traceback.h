@@ -3,6 +3,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "sw_strips.h"
+
 namespace gbsw {
 
 struct TraceParams {
@@ -31,6 +33,8 @@ struct TraceParams {
     int32_t* nops;               // per pair: operations written
     int32_t* path_score;         // per pair: H(k, m) of the path
     int* error;
+    int* queue;                  // int16 kernel: work-queue counter (0 before the launch)
+    int neg, top;                // int16 kernel: Trace16Limits
 };
 
 // Error bit: a path's end value differs from the pair's score.
@@ -64,7 +68,57 @@ __host__ __device__ inline int64_t trace_dir_words(int m, int k) {
 }
 
 cudaError_t launch_trace(const TraceParams& p, cudaStream_t stream);
-// Copies pair k's nops[k] operations from its slot to out + out_off[k].
+
+// ---- the int16x2 kernel (trace_strips.cu) ----
+// Columns a virtual lane holds and columns of a strip.
+constexpr int kTrace16Cols = 4;
+constexpr int kTrace16Width = strip_width(kTrace16Cols);
+// The limits of its values, from the scoring (`best`: the largest score of an
+// aligned pair of symbols).  neg: its -inf, as low as the rows of the pipeline's
+// fill (131 at most, each up to |ext| lower than the one before) leave room for.
+// top: a cell may lie above its upper neighbour by up to best + |open|, so a kernel
+// that looks at every sixteenth row sees a value above top before one can wrap.
+struct Trace16Limits {
+    int neg, top, best;
+};
+inline Trace16Limits trace16_limits(int best, int open, int ext) {
+    return {-32768 - 131 * ext - open + 160, 32767 - 20 * (best - open), best};
+}
+
+// Threads of a walk block and lanes per walk.
+constexpr int kWalkThreads = 128;
+constexpr int kWalkLanes = 8;
+
+// Whether the scoring suits it: int8 scores, match at least mismatch and at most
+// 128 above it (DNA), open <= ext (the gap row then follows from the recurrence) and
+// small gaps.
+inline bool trace16_scores_ok(bool int8_scores, int match, int mismatch, bool protein, int open, int ext) {
+    return int8_scores && (protein || (match >= mismatch && match - mismatch <= 128)) && open <= ext && ext >= -16 && open >= -256;
+}
+// Whether a pair's segment does: every real value lies above -inf, and none above
+// top if the score is the pair's (a prefix of the path aligns two substrings, so no
+// value exceeds the best local score; results of other inputs are told from it by
+// the kernel's own look).
+inline bool trace16_pair_ok(const Trace16Limits& lim, int m, int k, int score, int open, int ext) {
+    return ((int64_t)lim.best * (m < k ? m : k) <= lim.top || score <= lim.top) &&
+           2 * (int64_t)open + (int64_t)ext * ((int64_t)m + k) >= lim.neg + 256;
+}
+// Direction words (32 bits) of a strip of `lanes` virtual lanes and `pairs` row pairs:
+// two per lane and step, steps rounded up to four.
+__host__ __device__ inline int64_t trace16_strip_words(int pairs, int lanes) {
+    return (int64_t)((pairs + lanes - 1 + 3) / 4) * 256;
+}
+// Direction words of a pair.
+inline int64_t trace16_dir_words(int m, int k) {
+    const int strips = (m + kTrace16Width - 1) / kTrace16Width, pairs = (k + 2) / 2;
+    const int lanes = (m - (strips - 1) * kTrace16Width + kTrace16Cols - 1) / kTrace16Cols;
+    return (strips - 1) * trace16_strip_words(pairs, 64) + trace16_strip_words(pairs, lanes);
+}
+cudaError_t trace16_occupancy(bool protein, int* blocks_per_sm);
+// The DP of `ntasks` strip tasks (s.tasks, a pair's strips one after another), then
+// the walks of the pairs p.order[0 .. p.count), their runs at the ends of their slots.
+cudaError_t launch_trace16(const TraceParams& p, const StripParams& s, int ntasks, int blocks, cudaStream_t stream);
+// Copies pair k's nops[k] operations from the end of its slot to out + out_off[k].
 cudaError_t launch_gather_ops(const uint32_t* ops, const int64_t* slot_off, const int32_t* nops,
                               const int64_t* out_off, uint32_t* out, int64_t n, cudaStream_t stream);
 
