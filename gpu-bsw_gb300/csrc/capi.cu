@@ -90,6 +90,7 @@ struct gbsw_context {
     DevBuf<int> d_hist;      // schedule: bucket counters / offsets, then the class ranges
     DevBuf<int> d_matrix;    // 25x25 (score - open)
     DevBuf<int> d_encoding;  // 91 entries
+    std::vector<int16_t> matrix_on_device;  // the scores d_matrix holds (empty: none)
     // strip-parallel passes: task list, edge buffers, read marks and the next unused tag
     DevBuf<int2> d_tasks;
     DevBuf<uint64_t> d_edges;
@@ -137,8 +138,12 @@ int check_scoring(gbsw_context* ctx, const gbsw_scoring* sc) {
 }
 
 // Upload the protein matrix (padded to 25x25 with a large negative row/column
-// for padding columns) and the encoding table.
+// for padding columns) and the encoding table, unless the device holds the same
+// scores already (compared value by value: two copies and a wait on the stream).
 int upload_protein_tables(gbsw_context* ctx, const gbsw_scoring* sc, cudaStream_t stream) {
+    if (ctx->matrix_on_device.size() == 576 && std::equal(sc->matrix, sc->matrix + 576, ctx->matrix_on_device.begin()))
+        return GBSW_OK;
+    ctx->matrix_on_device.clear();
     cudaError_t e = ctx->d_matrix.reserve(gbsw::kAADim * gbsw::kAADim);
     if (e == cudaSuccess) e = ctx->d_encoding.reserve(91);
     if (e != cudaSuccess) return ctx->cuda_fail(e, "cudaMalloc(protein tables)");
@@ -159,9 +164,11 @@ int upload_protein_tables(gbsw_context* ctx, const gbsw_scoring* sc, cudaStream_
         e = cudaMemcpyAsync(ctx->d_encoding.ptr, he, sizeof(int) * 91, cudaMemcpyHostToDevice,
                             stream);
     if (e != cudaSuccess) return ctx->cuda_fail(e, "cudaMemcpyAsync(protein tables)");
-    // the host copies above read pinned staging that the next call may rewrite
+    // the host copies above read pinned staging that the next call may rewrite, and
+    // the next call's stream may be another one
     e = cudaStreamSynchronize(stream);
     if (e != cudaSuccess) return ctx->cuda_fail(e, "cudaStreamSynchronize");
+    ctx->matrix_on_device.assign(sc->matrix, sc->matrix + 576);
     return GBSW_OK;
 }
 
@@ -348,7 +355,6 @@ int run_passes(gbsw_context* ctx, const gbsw_scoring* sc, const uint8_t* ref, co
         if (rc != GBSW_OK) return rc;
     }
     e = cudaMemsetAsync(ctx->d_misc.ptr, 0, sizeof(int) * 32, stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(ctx->d_rerun.ptr, 0, sizeof(int) * 2, stream);
     if (e != cudaSuccess) return ctx->cuda_fail(e, "cudaMemsetAsync");
 
     gbsw::SchedParams sp{};
@@ -377,18 +383,91 @@ int run_passes(gbsw_context* ctx, const gbsw_scoring* sc, const uint8_t* ref, co
     sp.order = ctx->d_order.ptr;
     sp.error = ctx->d_misc.ptr + 3;
 
+    const int rows = (std::max(1, max_len) + 1) & ~1;  // even: 16-byte boundary copies stay in a group's buffer
+    gbsw::PassParams p{};
+    p.ref = ref;
+    p.ref_off = ref_off;
+    p.query = query;
+    p.query_off = query_off;
+    p.n = n;
+    p.open = sc->gap_open;
+    p.ext = sc->gap_extend;
+    p.match = sc->match;
+    p.mismatch = sc->mismatch;
+    p.aa_matrix = ctx->d_matrix.ptr;
+    p.aa_encoding = ctx->d_encoding.ptr;
+    p.score = score;
+    p.ref_begin = ref_begin;
+    p.ref_end = ref_end;
+    p.query_begin = query_begin;
+    p.query_end = query_end;
+    p.order = sp.order;
+    p.class_range = sp.class_range;
+    p.scratch_rows = rows;
+    p.error = ctx->d_misc.ptr + 3;
+    p.rev_p = rev_p;
+    // the dual-pair passes stay exact while every H is at most 32767 - match_pos
+    // (sw_dual.cu); a pair whose best exceeds it is rerun in int32
+    p.dual_limit = 32767 - match_pos;
+    p.rerun = ctx->d_rerun.ptr;
+    p.pair_cls = ctx->d_cls.ptr;
+
+    // Strip-parallel tasks of `pairs` pairs at most, and whether 8 columns a lane
+    // serve them: once the long pairs alone give every scheduler several strips of
+    // 4 the steps' fixed work counts, not the chain of one strip (3,000 mixed pairs,
+    // 900 of them long, 1,435 against 1,502 us forward, 300 long reads 7.27 against
+    // 8.17 ms; below that 4 win: 61 long reads 2.35 against 2.50 ms, 1,000 mixed
+    // pairs 746 against 801 us).
+    auto strip_tasks = [&](int64_t pairs, int cols) {
+        return pairs * ((std::max(1, max_len) + gbsw::strip_width(cols) - 1) / gbsw::strip_width(cols));
+    };
+    auto wide_strips = [&](int64_t long_pairs) {
+        return !protein && max_len >= gbsw::kLongCols && strip_tasks(long_pairs, 4) >= 8192;
+    };
+    // A small batch whose plan is block per pair whatever its bins hold: one block
+    // schedules it, and nothing waits for the counts (unless they choose the strips'
+    // width).
+    bool small = !tune && plan.binned && n <= gbsw::kSmallSchedule;
+    for (int b = 0; small && b < gbsw::kBins; ++b) {
+        auto team = [&](const gbsw_variant& v) { return !v.dual && v.lanes == gbsw::kTeamLanes; };
+        if (!use_table) {
+            small = team(plan.bin[0][b]) && team(plan.bin[1][b]);
+            continue;
+        }
+        for (int k = 0; small && k <= count_bucket(n); ++k) {
+            const gbsw_variant& rv = table.reverse[sc->kind][b][k];
+            small = team(table.variant[sc->kind][b][k]) && (team(rv) || !variant_ok(protein, rv, dual_ok));
+        }
+    }
+    gbsw::StripParams strip_params{};
     cudaEventRecord(ctx->ev[EV_H2D], stream);
-    e = gbsw::build_schedule(sp, false, ctx->sms, stream);
+    const bool ask_counts = !small || wide_strips(n);
+    if (small) {
+        if (use_table)
+            for (int b = 0; b < gbsw::kBins; ++b) {
+                plan.bin[0][b] = plan.bin[1][b] = gbsw_variant{0, gbsw::kTeamLanes};
+                plan.from_table[b] = true;
+            }
+        int rc = reserve_strips(ctx, strip_tasks(n, 4), 4 * strip_tasks(n, 4), rows, stream, &strip_params);
+        if (rc != GBSW_OK) return rc;
+        sp.classes_only = 1;
+        e = gbsw::classify_pairs(sp, ctx->sms, stream);
+        if (e == cudaSuccess)
+            e = gbsw::launch_small_schedule(false, p, strip_params, sp.order, sp.class_range, ask_counts ? 0 : 4, stream);
+    } else {
+        e = cudaMemsetAsync(ctx->d_rerun.ptr, 0, sizeof(int) * 2, stream);
+        if (e == cudaSuccess) e = gbsw::build_schedule(sp, false, ctx->sms, stream);
+    }
     if (e != cudaSuccess) return ctx->cuda_fail(e, "schedule");
-    int launches = 3;
+    int launches = small ? 2 : 3;
     ctx->stats.bin_pairs[0] = ctx->stats.bin_pairs[1] = -1;
     // pairs of each range of the forward schedule, when read back (else -1:
     // unknown, launch anyway)
     int64_t range_pairs[gbsw::kRanges];
     for (int64_t& c : range_pairs) c = -1;
-    // (reading the counts back also tells which ranges are empty: skipping
-    // their launches saves more than the copy's wait costs, even on batches
-    // whose plan the counts cannot change -- 1,000 pairs: 0.235 against 0.253 ms).
+    // every pair the int16x2 kernels may take went to a bin
+    if (plan.binned) range_pairs[0] = 0;
+    // Reading the counts back also tells which ranges are empty.
     // A caller that knows the bins' counts on the host (the serving loop) skips
     // the wait: the plan comes from its counts, a bin it counts empty is empty on
     // the device too, and the other ranges launch whatever they hold.
@@ -413,13 +492,15 @@ int run_passes(gbsw_context* ctx, const gbsw_scoring* sc, const uint8_t* ref, co
         if (variant_ok(protein, rv, dual_ok)) plan.bin[1][b] = rv;
         plan.from_table[b] = true;
     };
-    if (host_bins && use_table && !tune) {
+    if (!ask_counts) {
+        // nothing to ask
+    } else if (host_bins && use_table && !tune) {
         for (int b = 0; b < gbsw::kBins; ++b) {
             const int64_t count = std::max<int64_t>(0, host_bins[b]);
             range_pairs[b ? gbsw::kRangeLong : gbsw::kRangeShort] = count;
             take_count(b, count);
         }
-    } else if (use_table || tune) {
+    } else if (use_table || tune || small) {
         int* hr = ctx->h_misc.ptr + 32;
         e = cudaMemcpyAsync(hr, sp.class_range, sizeof(int) * 2 * gbsw::kRanges, cudaMemcpyDeviceToHost, stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
@@ -429,25 +510,15 @@ int run_passes(gbsw_context* ctx, const gbsw_scoring* sc, const uint8_t* ref, co
     }
 
     // block-per-pair plans of the binned pairs run strip-parallel in int16x2
-    const int rows = (std::max(1, max_len) + 1) & ~1;  // even: 16-byte boundary copies stay in a group's buffer
-    auto strip_tasks = [&](int64_t pairs, int cols) {
-        return pairs * ((std::max(1, max_len) + gbsw::strip_width(cols) - 1) / gbsw::strip_width(cols));
-    };
-    // 8 columns a lane once the long pairs alone give every scheduler several strips
-    // of 4 (then the steps' fixed work counts, not the chain of one strip): 3,000 mixed
-    // pairs, 900 of them long, 1,435 against 1,502 us forward, 300 long reads 7.27
-    // against 8.17 ms; below that 4 win: 61 long reads 2.35 against 2.50 ms, 1,000
-    // mixed pairs 746 against 801 us.
     const int64_t long_pairs = range_pairs[gbsw::kRangeLong] >= 0 ? range_pairs[gbsw::kRangeLong] : n;
-    const int strip_cols = gbsw::strip_columns(protein, strip_tasks(long_pairs, 4) >= 8192);
+    const int strip_cols = gbsw::strip_columns(protein, wide_strips(long_pairs));
     const int64_t strip_bound = strip_tasks(n, strip_cols);
     const bool strips_fit = plan.binned && strip_bound <= kMaxStripTasks;
     auto strips = [&](int rev, int b) {
         return strips_fit && !plan.bin[rev][b].dual && plan.bin[rev][b].lanes == gbsw::kTeamLanes;
     };
     const bool any_strips[2] = {strips(0, 0) || strips(0, 1), strips(1, 0) || strips(1, 1)};
-    gbsw::StripParams strip_params{};
-    if (any_strips[0] || any_strips[1]) {
+    if (!small && (any_strips[0] || any_strips[1])) {
         int rc = reserve_strips(ctx, strip_bound, 4 * strip_bound, rows, stream, &strip_params);
         if (rc != GBSW_OK) return rc;
     }
@@ -498,34 +569,7 @@ int run_passes(gbsw_context* ctx, const gbsw_scoring* sc, const uint8_t* ref, co
     e = ctx->d_scratch.reserve((size_t)groups * (size_t)rows);
     if (e != cudaSuccess) return ctx->fail(GBSW_ENOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
 
-    gbsw::PassParams p{};
-    p.ref = ref;
-    p.ref_off = ref_off;
-    p.query = query;
-    p.query_off = query_off;
-    p.n = n;
-    p.open = sc->gap_open;
-    p.ext = sc->gap_extend;
-    p.match = sc->match;
-    p.mismatch = sc->mismatch;
-    p.aa_matrix = ctx->d_matrix.ptr;
-    p.aa_encoding = ctx->d_encoding.ptr;
-    p.score = score;
-    p.ref_begin = ref_begin;
-    p.ref_end = ref_end;
-    p.query_begin = query_begin;
-    p.query_end = query_end;
-    p.order = sp.order;
-    p.class_range = sp.class_range;
     p.scratch = ctx->d_scratch.ptr;
-    p.scratch_rows = rows;
-    p.error = ctx->d_misc.ptr + 3;
-    p.rev_p = rev_p;
-    // the dual-pair passes stay exact while every H is at most 32767 - match_pos
-    // (sw_dual.cu); a pair whose best exceeds it is rerun in int32
-    p.dual_limit = 32767 - match_pos;
-    p.rerun = ctx->d_rerun.ptr;
-    p.pair_cls = ctx->d_cls.ptr;
 
     // class launches, each bracketed by events when tuning
     auto timed = [&](int rev, int cls, auto&& launch) -> cudaError_t {
@@ -538,7 +582,9 @@ int run_passes(gbsw_context* ctx, const gbsw_scoring* sc, const uint8_t* ref, co
     // takes no pair whose score may exceed int16 (reverse_keys sends those to
     // class 0)
     const bool any_dual = plan.any_dual(0) || plan.any_dual(1);
-    const bool any_int16 = any_dual || any_strips[0] || any_strips[1];
+    // no score of these pairs can pass the int16x2 limit: nothing to rerun
+    const bool may_rerun = (int64_t)match_pos * rows > p.dual_limit;
+    const bool any_int16 = (any_dual || any_strips[0] || any_strips[1]) && may_rerun;
     // A range known to be empty needs no launch.  A pair keeps its forward
     // range in the reverse pass, except pairs with no score (to the idle class)
     // and dual-pair pairs rerun in int32 (to class 0), so class 0's reverse
@@ -552,9 +598,10 @@ int run_passes(gbsw_context* ctx, const gbsw_scoring* sc, const uint8_t* ref, co
             sp.rev_dual_bins = plan.binned ? (plan.bin[1][0].dual || strips(1, 0) ? 1 : 0) |
                                                  (plan.bin[1][1].dual || strips(1, 1) ? 2 : 0)
                                            : 0;
-            e = gbsw::build_schedule(sp, true, ctx->sms, stream);
+            e = small ? gbsw::launch_small_schedule(true, p, strip_params, sp.order, sp.class_range, strip_cols, stream)
+                      : gbsw::build_schedule(sp, true, ctx->sms, stream);
             if (e != cudaSuccess) return ctx->cuda_fail(e, "schedule");
-            launches += 3;
+            launches += small ? 1 : 3;
         }
         auto queue = [&](int cls) { return ctx->d_misc.ptr + (rev ? 16 : 8) + cls; };
         if (plan.binned) {
@@ -574,8 +621,10 @@ int run_passes(gbsw_context* ctx, const gbsw_scoring* sc, const uint8_t* ref, co
                     if (strips(rev, b)) {
                         strip_params.tag_base = ctx->strip_tag;
                         ctx->strip_tag += (unsigned)strip_bound;
-                        ++launches;
-                        return gbsw::launch_strips(rev != 0, protein, strip_cols, p, strip_params, grid[rev][cls], stream);
+                        const bool list = !small || (!rev && ask_counts);
+                        launches += list;
+                        return gbsw::launch_strips(rev != 0, protein, strip_cols, list, p, strip_params, grid[rev][cls],
+                                                   stream);
                     }
                     return v.dual ? gbsw::launch_pass_dual(rev != 0, protein, v.lanes, p, grid[rev][cls], stream)
                                   : gbsw::launch_pass(score_mode(sc, 0, dna_profile_ok, aa_profile_ok), rev != 0, dpx,
@@ -589,12 +638,14 @@ int run_passes(gbsw_context* ctx, const gbsw_scoring* sc, const uint8_t* ref, co
             if (empty(rev, cls)) continue;
             p.cls = cls;
             p.queue = queue(cls);
+            // no more blocks than pairs of its own (a team's block takes one at a time)
+            const int blocks = plan.int32_lanes == gbsw::kTeamLanes ? (int)std::min<int64_t>(grid[rev][cls], n) : grid[rev][cls];
             e = gbsw::launch_pass(score_mode(sc, cls, dna_profile_ok, aa_profile_ok), rev != 0, dpx, plan.int32_lanes,
-                                  p, grid[rev][cls], stream);
+                                  p, blocks, stream);
             if (e != cudaSuccess) return ctx->cuda_fail(e, rev ? "reverse pass launch" : "forward pass launch");
             ++launches;
         }
-        if ((plan.any_dual(0) || any_strips[0]) && !rev) {
+        if ((plan.any_dual(0) || any_strips[0]) && may_rerun && !rev) {
             // the dual-pair pairs that may have overflowed int16, in the int32
             // class-0 kernel: its work list is the rerun list the dual launches
             // above filled (class range [rerun[0], rerun[1]) = [0, count))
@@ -613,7 +664,7 @@ int run_passes(gbsw_context* ctx, const gbsw_scoring* sc, const uint8_t* ref, co
     ctx->stats.launches = launches;
     ctx->stats.lane_group = plan.binned ? plan.bin[0][0].lanes : plan.int32_lanes;
     ctx->stats.dual = any_dual ? 1 : 0;
-    ctx->stats.reruns = plan.any_dual(0) || any_strips[0] ? -1 : 0;  // read back on demand (gbsw_last_stats)
+    ctx->stats.reruns = (plan.any_dual(0) || any_strips[0]) && may_rerun ? -1 : 0;  // read back on demand (gbsw_last_stats)
     for (int b = 0; b < gbsw::kBins; ++b) {
         ctx->stats.bin_dual[b] = plan.binned ? plan.bin[0][b].dual : 0;
         ctx->stats.bin_lanes[b] = plan.binned ? plan.bin[0][b].lanes : plan.int32_lanes;

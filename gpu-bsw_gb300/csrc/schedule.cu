@@ -121,8 +121,9 @@ __global__ void forward_keys(SchedParams s) {
             if (cls == 0 && s.binned) cls = ncols >= kLongCols ? kClassLong : kClassShort;
             // bins: strips then rows, which pairs like shapes for the two-pair
             // units and is longest-first for one-pair plans as well
-            const int key = pair_key(cls, nrows, ncols);
             s.cls[k] = (uint8_t)cls;
+            if (s.classes_only) continue;
+            const int key = pair_key(cls, nrows, ncols);
             s.keys[k] = key;
             atomicAdd(&s.hist[key], 1);
         }
@@ -220,6 +221,11 @@ int grid_for(int64_t items, int per_block, int sms) {
 }
 
 }  // namespace
+
+cudaError_t classify_pairs(const SchedParams& s, int sms, cudaStream_t stream) {
+    forward_keys<<<grid_for(s.n * 32, kKeyThreads, sms), kKeyThreads, 0, stream>>>(s);
+    return cudaGetLastError();
+}
 
 cudaError_t build_schedule(const SchedParams& s, bool reverse, int sms, cudaStream_t stream) {
     cudaError_t e = cudaMemsetAsync(s.hist, 0, sizeof(int) * kBuckets, stream);

@@ -30,8 +30,11 @@ struct SchedParams {
     int* class_range;     // 2 * kRanges ints: [begin, end) of each class, then of the two bins
     int* order;           // n pair indices in schedule order
     int* error;
+    int classes_only;     // forward keys: write the classes and nothing else
 };
 
+// Enqueues the classes of the pairs alone (s.classes_only set).
+cudaError_t classify_pairs(const SchedParams& s, int sms, cudaStream_t stream);
 // Enqueues the schedule kernels of one pass on `stream`.
 cudaError_t build_schedule(const SchedParams& s, bool reverse, int sms, cudaStream_t stream);
 

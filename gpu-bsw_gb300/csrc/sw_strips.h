@@ -35,9 +35,18 @@ __host__ __device__ constexpr int strip_width(int columns) { return 64 * columns
 // Columns a lane holds: 8 where there is a kernel for them and `wide` is asked for.
 inline int strip_columns(bool aa, bool wide) { return wide && !aa ? 8 : 4; }
 
+// Most pairs of the one-block schedule below.
+constexpr int kSmallSchedule = 4096;
+// Orders up to kSmallSchedule pairs whose binned ones all run strip by strip: their
+// classes (p.pair_cls; reverse: those above p.dual_limit take class 0), each by
+// descending cost, into p.order and p.class_range (writable copies of the
+// pointers), lists the strips of the binned ones (`columns` a lane; 0: none) and
+// clears the rerun count.
+cudaError_t launch_small_schedule(bool reverse, const PassParams& p, const StripParams& s, int* order, int* class_range,
+                                  int columns, cudaStream_t stream);
 cudaError_t strips_occupancy(bool reverse, bool aa, int columns, int* blocks_per_sm);
-// Lists the strips of range p.cls of the schedule, then runs them.
-cudaError_t launch_strips(bool reverse, bool aa, int columns, const PassParams& p, const StripParams& s, int blocks,
-                          cudaStream_t stream);
+// Runs the strips of range p.cls of the schedule, after listing them if `list`.
+cudaError_t launch_strips(bool reverse, bool aa, int columns, bool list, const PassParams& p, const StripParams& s,
+                          int blocks, cudaStream_t stream);
 
 }  // namespace gbsw
