@@ -97,6 +97,9 @@ struct gbsw_context {
     DevBuf<unsigned> d_freed;
     unsigned strip_tag = 1;
     HostBuf<int> h_misc;
+    // host entries, small calls: the inputs side by side, and the results
+    HostBuf<uint8_t> h_in, h_out;
+    DevBuf<uint8_t> d_in;
     // traceback
     DevBuf<uint32_t> d_tb_ops, d_tb_dir, d_tb_out;
     DevBuf<int2> d_tb_bnd;
@@ -312,7 +315,7 @@ int run_passes(gbsw_context* ctx, const gbsw_scoring* sc, const uint8_t* ref, co
                const uint8_t* query, const int64_t* query_off, int64_t n, int max_len,
                int32_t* score, int32_t* ref_begin, int32_t* ref_end, int32_t* query_begin,
                int32_t* query_end, cudaStream_t stream, const gbsw_variant* tune = nullptr,
-               const int64_t* host_bins = nullptr) {
+               const int64_t* host_bins = nullptr, bool no_raw = false) {
     const bool protein = sc->kind == GBSW_PROTEIN;
     const bool dpx = ctx->opts.use_dpx != 0;
     const bool dna_profile_ok = !protein && fits_int8(sc->match) && fits_int8(sc->mismatch);
@@ -589,7 +592,9 @@ int run_passes(gbsw_context* ctx, const gbsw_scoring* sc, const uint8_t* ref, co
     // range in the reverse pass, except pairs with no score (to the idle class)
     // and dual-pair pairs rerun in int32 (to class 0), so class 0's reverse
     // launch stays whenever a dual launch could have queued reruns.
+    // `no_raw`: the caller knows that no pair holds anything but A/C/G/T.
     auto empty = [&](int rev, int range) {
+        if (range == 1 && no_raw && dna_profile_ok) return true;
         if (range_pairs[range] != 0) return false;
         return !(rev && range == 0 && any_int16);
     };
@@ -1111,6 +1116,9 @@ size_t packed_device_bytes(int kind, const gbsw_packed& p) {
     return b;
 }
 
+// Bytes of inputs and of results up to which a host call goes through staging.
+constexpr size_t kStagedIn = 64 << 10, kStagedOut = 256 << 10;
+
 template <typename T>
 int align_host(gbsw_context* ctx, const gbsw_scoring* sc, const HostSeqs& in, const int64_t* ref_off,
                const int64_t* query_off, int64_t n, T* ref_begin, T* ref_end, T* query_begin, T* query_end,
@@ -1147,18 +1155,44 @@ int align_host(gbsw_context* ctx, const gbsw_scoring* sc, const HostSeqs& in, co
     cudaError_t e = cudaSetDevice(ctx->device);
     if (e != cudaSuccess) return ctx->cuda_fail(e, "cudaSetDevice");
     cudaStream_t stream = ctx->stream;
-    e = ctx->d_ref.reserve((size_t)std::max<int64_t>(ra, 1));
-    if (e == cudaSuccess) e = ctx->d_query.reserve((size_t)std::max<int64_t>(qa, 1));
-    if (e == cudaSuccess) e = ctx->d_ref_off.reserve((size_t)n + 1);
-    if (e == cudaSuccess) e = ctx->d_query_off.reserve((size_t)n + 1);
+    // Small calls go through page-locked staging: the four inputs in one copy, and
+    // the five result arrays back in one (a copy from or to pageable memory is
+    // staged by the driver, each result array with a wait of its own: 16 reads of
+    // 100-150 bp 177 against 110 us).
+    auto up16 = [](size_t b) { return (b + 15) & ~(size_t)15; };
+    const size_t off_bytes = sizeof(int64_t) * (size_t)(n + 1);
+    const size_t at_qoff = up16(off_bytes), at_ref = 2 * at_qoff, at_query = at_ref + up16((size_t)ra),
+                 in_bytes = at_query + up16((size_t)qa);
+    const bool staged_in = !in.packed() && in_bytes <= kStagedIn;
+    const bool staged_out = sizeof(T) * 5 * (size_t)n <= kStagedOut;
+    if (staged_in) {
+        e = ctx->d_in.reserve(in_bytes);
+        if (e == cudaSuccess) e = ctx->h_in.reserve(in_bytes);
+    } else {
+        e = ctx->d_ref.reserve((size_t)std::max<int64_t>(ra, 1));
+        if (e == cudaSuccess) e = ctx->d_query.reserve((size_t)std::max<int64_t>(qa, 1));
+        if (e == cudaSuccess) e = ctx->d_ref_off.reserve((size_t)n + 1);
+        if (e == cudaSuccess) e = ctx->d_query_off.reserve((size_t)n + 1);
+    }
+    if (e == cudaSuccess && staged_out) e = ctx->h_out.reserve(sizeof(T) * 5 * (size_t)n);
     // int32 results, then (int16 form) their narrowed copy: 5n int32 + 5n int16
     if (e == cudaSuccess) e = ctx->d_results.reserve((size_t)n * 5 + (sizeof(T) < 4 ? ((size_t)n * 5 + 1) / 2 : 0));
     if (e == cudaSuccess && in.packed())
         e = ctx->d_pack.reserve(packed_device_bytes(sc->kind, *in.pref) + packed_device_bytes(sc->kind, *in.pquery));
     if (e != cudaSuccess) return ctx->fail(GBSW_ENOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+    const uint8_t* const dev_ref = staged_in ? ctx->d_in.ptr + at_ref : ctx->d_ref.ptr;
+    const uint8_t* const dev_query = staged_in ? ctx->d_in.ptr + at_query : ctx->d_query.ptr;
+    const int64_t* const dev_ref_off = staged_in ? (const int64_t*)ctx->d_in.ptr : ctx->d_ref_off.ptr;
+    const int64_t* const dev_query_off = staged_in ? (const int64_t*)(ctx->d_in.ptr + at_qoff) : ctx->d_query_off.ptr;
 
     cudaEventRecord(ctx->ev[EV_START], stream);
-    if (in.packed()) {
+    if (staged_in) {
+        std::memcpy(ctx->h_in.ptr, ref_off, off_bytes);
+        std::memcpy(ctx->h_in.ptr + at_qoff, query_off, off_bytes);
+        if (ra > 0) std::memcpy(ctx->h_in.ptr + at_ref, in.ref, (size_t)ra);
+        if (qa > 0) std::memcpy(ctx->h_in.ptr + at_query, in.query, (size_t)qa);
+        e = cudaMemcpyAsync(ctx->d_in.ptr, ctx->h_in.ptr, in_bytes, cudaMemcpyHostToDevice, stream);
+    } else if (in.packed()) {
         size_t used = 0, used_q = 0;
         e = upload_packed(ctx, sc->kind, *in.pref, 0, ctx->d_ref.ptr, stream, &used);
         if (e == cudaSuccess) e = upload_packed(ctx, sc->kind, *in.pquery, used, ctx->d_query.ptr, stream, &used_q);
@@ -1168,10 +1202,10 @@ int align_host(gbsw_context* ctx, const gbsw_scoring* sc, const HostSeqs& in, co
         if (e == cudaSuccess && qa > 0)
             e = cudaMemcpyAsync(ctx->d_query.ptr, in.query, (size_t)qa, cudaMemcpyHostToDevice, stream);
     }
-    if (e == cudaSuccess)
+    if (e == cudaSuccess && !staged_in)
         e = cudaMemcpyAsync(ctx->d_ref_off.ptr, ref_off, sizeof(int64_t) * (size_t)(n + 1),
                             cudaMemcpyHostToDevice, stream);
-    if (e == cudaSuccess)
+    if (e == cudaSuccess && !staged_in)
         e = cudaMemcpyAsync(ctx->d_query_off.ptr, query_off, sizeof(int64_t) * (size_t)(n + 1),
                             cudaMemcpyHostToDevice, stream);
     if (e != cudaSuccess) return ctx->cuda_fail(e, "cudaMemcpyAsync H2D");
@@ -1184,9 +1218,10 @@ int align_host(gbsw_context* ctx, const gbsw_scoring* sc, const HostSeqs& in, co
     }
 
     int32_t* R = ctx->d_results.ptr;
-    rc = run_passes(ctx, sc, ctx->d_ref.ptr, ctx->d_ref_off.ptr, ctx->d_query.ptr,
-                    ctx->d_query_off.ptr, n, max_len, R, R + n, R + 2 * n, R + 3 * n, R + 4 * n,
-                    stream);
+    // a packed stream without escapes holds only A/C/G/T
+    const bool no_raw = in.packed() && in.pref->nruns == 0 && in.pquery->nruns == 0;
+    rc = run_passes(ctx, sc, dev_ref, dev_ref_off, dev_query, dev_query_off, n, max_len, R, R + n, R + 2 * n, R + 3 * n,
+                    R + 4 * n, stream, nullptr, nullptr, no_raw);
     if (rc != GBSW_OK) return rc;
     // results straight into the caller's five arrays (narrowed on the device first)
     const T* D = reinterpret_cast<const T*>(R);
@@ -1199,7 +1234,9 @@ int align_host(gbsw_context* ctx, const gbsw_scoring* sc, const HostSeqs& in, co
         D = d16;
     }
     T* outs[5] = {top_scores, ref_begin, ref_end, query_begin, query_end};
-    for (int f = 0; f < 5 && e == cudaSuccess; ++f)
+    if (staged_out && e == cudaSuccess)
+        e = cudaMemcpyAsync(ctx->h_out.ptr, D, sizeof(T) * 5 * (size_t)n, cudaMemcpyDeviceToHost, stream);
+    for (int f = 0; f < 5 && e == cudaSuccess && !staged_out; ++f)
         e = cudaMemcpyAsync(outs[f], D + (size_t)f * (size_t)n, sizeof(T) * (size_t)n, cudaMemcpyDeviceToHost,
                             stream);
     if (e == cudaSuccess) {
@@ -1211,6 +1248,9 @@ int align_host(gbsw_context* ctx, const gbsw_scoring* sc, const HostSeqs& in, co
     cudaEventRecord(ctx->ev[EV_D2H], stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
     if (e != cudaSuccess) return ctx->cuda_fail(e, "alignment");
+    if (staged_out)
+        for (int f = 0; f < 5; ++f)
+            std::memcpy(outs[f], ctx->h_out.ptr + sizeof(T) * (size_t)f * (size_t)n, sizeof(T) * (size_t)n);
     rc = decode_device_error(ctx, ctx->h_misc.ptr[0]);
     if (rc != GBSW_OK) return rc;
     ctx->timed_host = true;
@@ -1303,6 +1343,9 @@ void gbsw_destroy(gbsw_context* ctx) {
     ctx->d_order.release();
     ctx->d_hist.release();
     ctx->h_misc.release();
+    ctx->h_in.release();
+    ctx->h_out.release();
+    ctx->d_in.release();
     ctx->d_tb_ops.release();
     ctx->d_tb_dir.release();
     ctx->d_tb_out.release();
