@@ -308,6 +308,10 @@ int reserve_strips(gbsw_context* ctx, int64_t tasks, int64_t tags, int rows, cud
     return GBSW_OK;
 }
 
+// Boundary entries (8 bytes) up to which the launches of a pass get buffers of
+// their own and run beside one another.
+constexpr int64_t kBesideEntries = int64_t(1) << 27;
+
 // Enqueue the schedule and both passes for n pairs already on the device.
 // `tune` (gbsw_tune_device) forces every bin to one variant and times each
 // class launch with events; the result arrays are those of a normal call.
@@ -526,61 +530,12 @@ int run_passes(gbsw_context* ctx, const gbsw_scoring* sc, const uint8_t* ref, co
         if (rc != GBSW_OK) return rc;
     }
     // their int16 overflows are long pairs: rerun block per pair
+    const int raw_lanes = plan.int32_lanes;
     if (any_strips[0]) plan.int32_lanes = gbsw::kTeamLanes;
 
     // the bins share one launch over their whole class when their plans agree
     // (the tuner times them apart)
     auto merged = [&](int rev) { return !tune && plan.merged(rev); };
-    // persistent grids: each launch fills the SMs to its variant's occupancy
-    // (gbsw_options.blocks_per_sm > 0 overrides); the boundary scratch holds one
-    // buffer per group of the largest launch
-    int grid[2][gbsw::kRanges] = {};
-    int64_t groups = 0;
-    for (int rev = 0; rev < 2; ++rev) {
-        for (int cls = 0; cls < nclasses; ++cls) {
-            int rc = dual_or_pass_occupancy(ctx, protein, score_mode(sc, cls, dna_profile_ok, aa_profile_ok), rev != 0,
-                                            dpx, gbsw_variant{0, plan.int32_lanes}, &grid[rev][cls]);
-            if (rc != GBSW_OK) return rc;
-            groups = std::max(groups, (int64_t)grid[rev][cls] * gbsw::pass_groups_per_block(plan.int32_lanes));
-        }
-        if (plan.binned) {
-            for (int b = 0; b < gbsw::kBins; ++b) {
-                const int cls = b ? gbsw::kRangeLong : gbsw::kRangeShort;
-                const gbsw_variant& v = plan.bin[rev][b];
-                if (strips(rev, b)) {
-                    // a warp per task, spread over the SMs before they stack up
-                    int per_sm = ctx->opts.blocks_per_sm;
-                    if (per_sm <= 0) {
-                        e = gbsw::strips_occupancy(rev != 0, protein, strip_cols, &per_sm);
-                        if (e != cudaSuccess) return ctx->cuda_fail(e, "occupancy");
-                    }
-                    const int64_t want = (strip_bound + 3) / 4;
-                    per_sm = std::min(per_sm, 3);
-                    grid[rev][cls] = (int)std::min<int64_t>((int64_t)ctx->sms * std::max(1, per_sm),
-                                                            std::max<int64_t>(ctx->sms, want));
-                    continue;
-                }
-                int rc = dual_or_pass_occupancy(ctx, protein, score_mode(sc, 0, dna_profile_ok, aa_profile_ok),
-                                                rev != 0, dpx, v, &grid[rev][cls]);
-                if (rc != GBSW_OK) return rc;
-                const int lanes = v.dual ? gbsw::dual_lanes(protein, v.lanes) : v.lanes;
-                groups = std::max(groups, (int64_t)grid[rev][cls] * gbsw::pass_groups_per_block(lanes));
-            }
-            grid[rev][gbsw::kClassBinned] = grid[rev][gbsw::kRangeShort];
-        }
-    }
-    e = ctx->d_scratch.reserve((size_t)groups * (size_t)rows);
-    if (e != cudaSuccess) return ctx->fail(GBSW_ENOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
-
-    p.scratch = ctx->d_scratch.ptr;
-
-    // class launches, each bracketed by events when tuning
-    auto timed = [&](int rev, int cls, auto&& launch) -> cudaError_t {
-        if (tune) cudaEventRecord(ctx->ev_cls[rev][cls][0], stream);
-        cudaError_t r = launch();
-        if (tune) cudaEventRecord(ctx->ev_cls[rev][cls][1], stream);
-        return r;
-    };
     // dual forward launches may queue int32 reruns; a dual reverse launch
     // takes no pair whose score may exceed int16 (reverse_keys sends those to
     // class 0)
@@ -598,6 +553,96 @@ int run_passes(gbsw_context* ctx, const gbsw_scoring* sc, const uint8_t* ref, co
         if (range_pairs[range] != 0) return false;
         return !(rev && range == 0 && any_int16);
     };
+    // The launches of a pass: bins that run strip by strip (their few blocks first, so
+    // that they spread over the SMs), raw bytes, the other bins (long first, or both at
+    // once), the int32 class.  Persistent grids: each fills the SMs to its variant's
+    // occupancy (gbsw_options.blocks_per_sm > 0 overrides).  The boundary scratch holds
+    // a buffer per group.
+    struct Launch {
+        int range;             // the class or bin it works on
+        int bin;               // -1: an int32 class
+        gbsw_variant v;
+        int blocks;
+        int64_t groups, at;    // boundary buffers, and the first of them
+    };
+    std::vector<Launch> pass_launches[2];
+    int64_t groups = 0, side_by_side = 0;
+    for (int rev = 0; rev < 2; ++rev) {
+        auto add = [&](int range, int bin, const gbsw_variant& v) -> int {
+            // a bin's empty launch stays in the tuner's report (0 ms)
+            if (!(tune && bin >= 0) && empty(rev, range)) return GBSW_OK;
+            Launch l{range, bin, v, 0, 0, 0};
+            if (bin >= 0 && strips(rev, bin)) {
+                // a warp per task, spread over the SMs before they stack up
+                int per_sm = ctx->opts.blocks_per_sm;
+                if (per_sm <= 0) {
+                    e = gbsw::strips_occupancy(rev != 0, protein, strip_cols, &per_sm);
+                    if (e != cudaSuccess) return ctx->cuda_fail(e, "occupancy");
+                }
+                const int64_t want = (strip_bound + 3) / 4;
+                per_sm = std::min(per_sm, 3);
+                l.blocks = (int)std::min<int64_t>((int64_t)ctx->sms * std::max(1, per_sm),
+                                                  std::max<int64_t>(ctx->sms, want));
+            } else {
+                int rc = dual_or_pass_occupancy(
+                    ctx, protein, score_mode(sc, bin >= 0 ? 0 : range, dna_profile_ok, aa_profile_ok), rev != 0, dpx, v,
+                    &l.blocks);
+                if (rc != GBSW_OK) return rc;
+                // no more blocks than pairs (a team's block takes one at a time)
+                if (!v.dual && v.lanes == gbsw::kTeamLanes) l.blocks = (int)std::min<int64_t>(l.blocks, n);
+                const int lanes = v.dual ? gbsw::dual_lanes(protein, v.lanes) : v.lanes;
+                l.groups = (int64_t)l.blocks * gbsw::pass_groups_per_block(lanes);
+            }
+            pass_launches[rev].push_back(l);
+            return GBSW_OK;
+        };
+        int rc = GBSW_OK;
+        auto add_bins = [&](bool strip_bins) {
+            if (!plan.binned) return;
+            if (merged(rev)) {
+                if (strips(rev, 0) == strip_bins) rc = add(gbsw::kClassBinned, 0, plan.bin[rev][0]);
+                return;
+            }
+            for (int b = gbsw::kBins - 1; b >= 0 && rc == GBSW_OK; --b)
+                if (strips(rev, b) == strip_bins)
+                    rc = add(b ? gbsw::kRangeLong : gbsw::kRangeShort, b, plan.bin[rev][b]);
+        };
+        add_bins(true);
+        if (rc == GBSW_OK && nclasses > 1) rc = add(1, -1, gbsw_variant{0, raw_lanes});
+        if (rc == GBSW_OK) add_bins(false);
+        if (rc == GBSW_OK) rc = add(0, -1, gbsw_variant{0, plan.int32_lanes});
+        if (rc != GBSW_OK) return rc;
+        int64_t sum = 0;
+        for (Launch& l : pass_launches[rev]) {
+            l.at = sum;
+            sum += l.groups;
+            groups = std::max(groups, l.groups);
+        }
+        side_by_side = std::max(side_by_side, sum);
+    }
+    // the rerun of int16x2 overflows is a launch of its own after the forward pass
+    int rerun_blocks = 0;
+    const bool rerun = (plan.any_dual(0) || any_strips[0]) && may_rerun;
+    if (rerun) {
+        int rc = dual_or_pass_occupancy(ctx, protein, score_mode(sc, 0, dna_profile_ok, aa_profile_ok), false, dpx,
+                                        gbsw_variant{0, plan.int32_lanes}, &rerun_blocks);
+        if (rc != GBSW_OK) return rc;
+        groups = std::max(groups, (int64_t)rerun_blocks * gbsw::pass_groups_per_block(plan.int32_lanes));
+    }
+    // Launches of one pass work on different pairs: with boundary buffers of their own
+    // they run beside one another, and the last wave of one is filled by the next.
+    const bool beside = !tune && side_by_side * rows <= kBesideEntries;
+    if (beside) groups = std::max(groups, side_by_side);
+    e = ctx->d_scratch.reserve((size_t)std::max<int64_t>(groups, 1) * (size_t)rows);
+    if (e != cudaSuccess) return ctx->fail(GBSW_ENOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+
+    // class launches, each bracketed by events when tuning
+    auto timed = [&](int rev, int cls, auto&& launch) -> cudaError_t {
+        if (tune) cudaEventRecord(ctx->ev_cls[rev][cls][0], stream);
+        cudaError_t r = launch();
+        if (tune) cudaEventRecord(ctx->ev_cls[rev][cls][1], stream);
+        return r;
+    };
     for (int rev = 0; rev < 2; ++rev) {
         if (rev) {
             sp.rev_dual_bins = plan.binned ? (plan.bin[1][0].dual || strips(1, 0) ? 1 : 0) |
@@ -608,59 +653,60 @@ int run_passes(gbsw_context* ctx, const gbsw_scoring* sc, const uint8_t* ref, co
             if (e != cudaSuccess) return ctx->cuda_fail(e, "schedule");
             launches += small ? 1 : 3;
         }
-        auto queue = [&](int cls) { return ctx->d_misc.ptr + (rev ? 16 : 8) + cls; };
-        if (plan.binned) {
-            // the long bin first: its units are the heaviest work; one launch over
-            // the whole class (long bin first in its order) when the plans agree
-            for (int b = gbsw::kBins - 1; b >= 0; --b) {
-                if (merged(rev) && b == 1) continue;
-                const int cls = merged(rev) ? gbsw::kClassBinned : (b ? gbsw::kRangeLong : gbsw::kRangeShort);
-                if (empty(rev, cls)) {
-                    if (tune) timed(rev, cls, [] { return cudaSuccess; });  // 0 ms for the report
-                    continue;
-                }
-                const gbsw_variant& v = plan.bin[rev][b];
-                p.cls = cls;
-                p.queue = queue(cls);
-                e = timed(rev, cls, [&] {
-                    if (strips(rev, b)) {
-                        strip_params.tag_base = ctx->strip_tag;
-                        ctx->strip_tag += (unsigned)strip_bound;
-                        const bool list = !small || (!rev && ask_counts);
-                        launches += list;
-                        return gbsw::launch_strips(rev != 0, protein, strip_cols, list, p, strip_params, grid[rev][cls],
-                                                   stream);
-                    }
-                    return v.dual ? gbsw::launch_pass_dual(rev != 0, protein, v.lanes, p, grid[rev][cls], stream)
-                                  : gbsw::launch_pass(score_mode(sc, 0, dna_profile_ok, aa_profile_ok), rev != 0, dpx,
-                                                      v.lanes, p, grid[rev][cls], stream);
-                });
-                if (e != cudaSuccess) return ctx->cuda_fail(e, rev ? "reverse pass launch" : "forward pass launch");
-                ++launches;
+        auto strip_launch = [&](const Launch& l) { return l.bin >= 0 && strips(rev, l.bin); };
+        auto list = [&](const Launch& l) -> cudaError_t {
+            p.cls = l.range;
+            ++launches;
+            return gbsw::launch_list_strips(rev != 0, strip_cols, p, strip_params, stream);
+        };
+        // the list of strips comes before any launch (the tuner's launches list their own)
+        const bool lists = !small || (!rev && ask_counts);
+        for (const Launch& l : pass_launches[rev])
+            if (!tune && lists && strip_launch(l)) {
+                e = list(l);
+                if (e != cudaSuccess) return ctx->cuda_fail(e, "strip list");
             }
-        }
-        for (int cls = 0; cls < nclasses; ++cls) {
-            if (empty(rev, cls)) continue;
-            p.cls = cls;
-            p.queue = queue(cls);
-            // no more blocks than pairs of its own (a team's block takes one at a time)
-            const int blocks = plan.int32_lanes == gbsw::kTeamLanes ? (int)std::min<int64_t>(grid[rev][cls], n) : grid[rev][cls];
-            e = gbsw::launch_pass(score_mode(sc, cls, dna_profile_ok, aa_profile_ok), rev != 0, dpx, plan.int32_lanes,
-                                  p, blocks, stream);
+        bool first = true;
+        for (const Launch& l : pass_launches[rev]) {
+            if (tune && l.bin >= 0 && empty(rev, l.range)) {
+                timed(rev, l.range, [] { return cudaSuccess; });
+                continue;
+            }
+            p.join = beside && !first ? 1 : 0;
+            first = false;
+            p.cls = l.range;
+            p.queue = ctx->d_misc.ptr + (rev ? 16 : 8) + l.range;
+            p.scratch = ctx->d_scratch.ptr + (beside ? l.at : 0) * rows;
+            e = timed(rev, l.range, [&]() -> cudaError_t {
+                if (strip_launch(l)) {
+                    if (tune) {
+                        cudaError_t r = list(l);
+                        if (r != cudaSuccess) return r;
+                    }
+                    strip_params.tag_base = ctx->strip_tag;
+                    ctx->strip_tag += (unsigned)strip_bound;
+                    return gbsw::launch_strips(rev != 0, protein, strip_cols, p, strip_params, l.blocks, stream);
+                }
+                return l.v.dual ? gbsw::launch_pass_dual(rev != 0, protein, l.v.lanes, p, l.blocks, stream)
+                                : gbsw::launch_pass(score_mode(sc, l.bin >= 0 ? 0 : l.range, dna_profile_ok, aa_profile_ok),
+                                                    rev != 0, dpx, l.v.lanes, p, l.blocks, stream);
+            });
             if (e != cudaSuccess) return ctx->cuda_fail(e, rev ? "reverse pass launch" : "forward pass launch");
             ++launches;
         }
-        if ((plan.any_dual(0) || any_strips[0]) && may_rerun && !rev) {
+        if (rerun && !rev) {
             // the dual-pair pairs that may have overflowed int16, in the int32
             // class-0 kernel: its work list is the rerun list the dual launches
             // above filled (class range [rerun[0], rerun[1]) = [0, count))
             gbsw::PassParams pr = p;
+            pr.join = 0;
             pr.cls = 0;
             pr.class_range = ctx->d_rerun.ptr;
             pr.order = ctx->d_rerun.ptr + 2;
             pr.queue = ctx->d_misc.ptr + 24;
+            pr.scratch = ctx->d_scratch.ptr;
             e = gbsw::launch_pass(score_mode(sc, 0, dna_profile_ok, aa_profile_ok), false, dpx, plan.int32_lanes, pr,
-                                  grid[0][0], stream);
+                                  rerun_blocks, stream);
             if (e != cudaSuccess) return ctx->cuda_fail(e, "int32 rerun launch");
             ++launches;
         }
@@ -669,7 +715,7 @@ int run_passes(gbsw_context* ctx, const gbsw_scoring* sc, const uint8_t* ref, co
     ctx->stats.launches = launches;
     ctx->stats.lane_group = plan.binned ? plan.bin[0][0].lanes : plan.int32_lanes;
     ctx->stats.dual = any_dual ? 1 : 0;
-    ctx->stats.reruns = (plan.any_dual(0) || any_strips[0]) && may_rerun ? -1 : 0;  // read back on demand (gbsw_last_stats)
+    ctx->stats.reruns = rerun ? -1 : 0;  // read back on demand (gbsw_last_stats)
     for (int b = 0; b < gbsw::kBins; ++b) {
         ctx->stats.bin_dual[b] = plan.binned ? plan.bin[0][b].dual : 0;
         ctx->stats.bin_lanes[b] = plan.binned ? plan.bin[0][b].lanes : plan.int32_lanes;

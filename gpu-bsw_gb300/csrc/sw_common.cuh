@@ -126,7 +126,33 @@ struct PassParams {
     int dual_limit;
     int* rerun;
     uint8_t* pair_cls;
+    // 1: this launch runs beside the one before it (launch_beside), and ends after it
+    int join;
 };
+
+// The launches of one pass that work on different pairs run beside one another: each
+// lets the next one start at once, and one that started so waits for the one before
+// it at its end, so that whatever follows it comes after both.
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void end_after_previous(const PassParams& p) {
+    if (p.join) asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+// Launches `fn`; `beside`: without waiting for the kernel before it in the stream
+// (which must call let_next_start, and `fn` end_after_previous).
+inline cudaError_t launch_beside(const void* fn, int blocks, int threads, void** args, size_t dyn, cudaStream_t stream,
+                                 bool beside) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = dyn;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = beside ? 1 : 0;
+    return cudaLaunchKernelExC(&cfg, fn, args);
+}
 
 // Error flag bits.
 constexpr int kErrSymbol = 1;    // protein byte outside the encoding table

@@ -207,6 +207,7 @@ template <bool REVERSE, bool AA, int G, int C>
 __global__ void __launch_bounds__(kThreads, AA ? GBSW_DUAL_MIN_BLOCKS
                                                : (REVERSE ? GBSW_DUAL_REV_DNA_MIN_BLOCKS : GBSW_DUAL_FWD_DNA_MIN_BLOCKS))
     sw_pass_dual(PassParams p) {
+    let_next_start();
     constexpr int W = G * C;
     static_assert(G >= 2 && G <= 32 && (G & (G - 1)) == 0 && C % 4 == 0 && C <= (AA ? 16 : 32),
                   "group geometry");
@@ -885,6 +886,7 @@ __global__ void __launch_bounds__(kThreads, AA ? GBSW_DUAL_MIN_BLOCKS
             }
         }
     }
+    end_after_previous(p);
 }
 
 }  // namespace
@@ -938,7 +940,7 @@ cudaError_t launch_pass_dual(bool reverse, bool aa, int width, const PassParams&
         if (e != cudaSuccess) return e;
     }
     void* args[] = {(void*)&p};
-    return cudaLaunchKernel(fn, dim3(blocks), dim3(kThreads), args, dyn, stream);
+    return launch_beside(fn, blocks, kThreads, args, dyn, stream, p.join != 0);
 }
 
 cudaError_t pass_dual_occupancy(bool reverse, bool aa, int width, int* blocks_per_sm) {

@@ -71,7 +71,7 @@ cudaError_t launch_pass(int score, bool reverse, bool dpx, int width, const Pass
         if (e != cudaSuccess) return e;
     }
     void* args[] = {(void*)&p};
-    return cudaLaunchKernel(fn, dim3(blocks), dim3(kThreads), args, dyn, stream);
+    return launch_beside(fn, blocks, kThreads, args, dyn, stream, p.join != 0);
 }
 
 }  // namespace gbsw

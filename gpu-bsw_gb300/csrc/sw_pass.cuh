@@ -154,6 +154,7 @@ constexpr int kTeamSpin = 1 << 24;
 
 template <int SCORE, bool REVERSE, bool DPX, int G, int C, int TEAM = 1>
 __global__ void __launch_bounds__(kThreads, min_blocks<SCORE>()) sw_pass(PassParams p) {
+    let_next_start();
     constexpr int W = G * C;
     static_assert(TEAM == 1 || (G == 32 && TEAM == kThreads / 32), "a team is every warp of the block");
     // pipeline steps per loop iteration; the row codes of the next iteration are
@@ -165,7 +166,7 @@ __global__ void __launch_bounds__(kThreads, min_blocks<SCORE>()) sw_pass(PassPar
     static_assert(G >= 2 && G <= 32 && (G & (G - 1)) == 0 && C % 4 == 0, "group geometry");
     constexpr int kProfBytes = kAAProfRows * W;  // protein strip profile of one group
     constexpr bool AA = SCORE == kScoreAaProfile || SCORE == kScoreAaWide;
-    constexpr bool kLowBand = REVERSE && TEAM == 1;
+    constexpr bool kLowBand = REVERSE && TEAM == 1 && SCORE != kScoreDnaRaw;
     // protein profile of each group's strip (dynamic shared memory, kProfBytes
     // per group): row e holds s'(e, column) for the W columns
     extern __shared__ __align__(16) int8_t sprof_dyn[];
@@ -234,8 +235,9 @@ __global__ void __launch_bounds__(kThreads, min_blocks<SCORE>()) sw_pass(PassPar
     int nrows = 0, ncols = 0, nstrips = 0, pad = 0, strip = 0, st = 0, nsteps = 0, rows = 0;
     int ncols_run = 0;                // columns computed (reverse: bounded, see reverse_columns)
     int band = -1;                    // reverse: the band of reverse_band (-1: every row)
-    // reverse: its other side, reverse_low_band (teams run their strips side by
-    // side, where it saves nothing and cost 3%: 5,000 DNA pairs 0.477 against 0.465 ms)
+    // reverse: its other side, reverse_low_band (not for teams, which run their strips
+    // side by side, where it saves nothing and cost 3%: 5,000 DNA pairs 0.477 against
+    // 0.465 ms, nor for raw bytes)
     int low = -1;
     bool rev = false;                 // read both sequences back to front (reverse pass)
     bool a_short = false;
@@ -394,8 +396,10 @@ __global__ void __launch_bounds__(kThreads, min_blocks<SCORE>()) sw_pass(PassPar
             f[c] = 0;
         }
         diag0 = open;
-        if constexpr (!kRowChecks) {
-            ho_out = open;  // what lane 0 hands on before its first step (rows i < 1 of lane 1)
+        if constexpr (!kRowChecks || TEAM > 1) {
+            // what lane 0 hands on before its first step (rows i < 1 of lane 1; teams: the
+            // rows above a reverse strip's band, where a warp's earlier pair left its values)
+            ho_out = open;
             e_out = 0;
         }
         m = 0;
@@ -775,6 +779,7 @@ __global__ void __launch_bounds__(kThreads, min_blocks<SCORE>()) sw_pass(PassPar
             }
         }
     }
+    end_after_previous(p);
 }
 
 template <int SCORE, bool REVERSE, bool DPX, int G, int C, int TEAM = 1>

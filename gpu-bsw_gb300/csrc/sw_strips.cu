@@ -151,6 +151,7 @@ __host__ __device__ constexpr size_t strip_row_bytes(int columns) {
 
 template <bool REVERSE, bool AA, int C>
 __global__ void __launch_bounds__(kThreads, 4) sw_strips(PassParams p, StripParams s) {
+    let_next_start();
     constexpr int W = strip_width(C);
     static_assert(C % 4 == 0 && kStripRows <= 32, "geometry");
     // what lane 0 takes in at each step of this and the next chunk: the edge words
@@ -537,6 +538,7 @@ __global__ void __launch_bounds__(kThreads, 4) sw_strips(PassParams p, StripPara
             write_result<REVERSE>(p, pid, pv, best);
         }
     }
+    end_after_previous(p);
 }
 
 // Inclusive scan over the block's 1,024 threads; every thread gets its sum, *total
@@ -690,23 +692,22 @@ cudaError_t launch_small_schedule(bool reverse, const PassParams& p, const Strip
     return cudaGetLastError();
 }
 
-cudaError_t launch_strips(bool reverse, bool aa, int columns, bool list, const PassParams& p, const StripParams& s,
-                          int blocks, cudaStream_t stream) {
-    cudaError_t e = cudaSuccess;
-    if (list) {
-        if (reverse)
-            list_strips<true><<<1, 1024, 0, stream>>>(p, s, strip_width(columns));
-        else
-            list_strips<false><<<1, 1024, 0, stream>>>(p, s, strip_width(columns));
-        e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
-    }
+cudaError_t launch_list_strips(bool reverse, int columns, const PassParams& p, const StripParams& s, cudaStream_t stream) {
+    if (reverse)
+        list_strips<true><<<1, 1024, 0, stream>>>(p, s, strip_width(columns));
+    else
+        list_strips<false><<<1, 1024, 0, stream>>>(p, s, strip_width(columns));
+    return cudaGetLastError();
+}
+
+cudaError_t launch_strips(bool reverse, bool aa, int columns, const PassParams& p, const StripParams& s, int blocks,
+                          cudaStream_t stream) {
     size_t dyn = 0;
     const void* fn = pick_strips(reverse, aa, columns, &dyn);
-    e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
     if (e != cudaSuccess) return e;
     void* args[] = {(void*)&p, (void*)&s};
-    return cudaLaunchKernel(fn, dim3(blocks), dim3(kThreads), args, dyn, stream);
+    return launch_beside(fn, blocks, kThreads, args, dyn, stream, p.join != 0);
 }
 
 }  // namespace gbsw

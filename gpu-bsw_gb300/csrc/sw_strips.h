@@ -45,8 +45,9 @@ constexpr int kSmallSchedule = 4096;
 cudaError_t launch_small_schedule(bool reverse, const PassParams& p, const StripParams& s, int* order, int* class_range,
                                   int columns, cudaStream_t stream);
 cudaError_t strips_occupancy(bool reverse, bool aa, int columns, int* blocks_per_sm);
-// Runs the strips of range p.cls of the schedule, after listing them if `list`.
-cudaError_t launch_strips(bool reverse, bool aa, int columns, bool list, const PassParams& p, const StripParams& s,
-                          int blocks, cudaStream_t stream);
+// Lists the strips of range p.cls of the schedule, and runs the listed ones.
+cudaError_t launch_list_strips(bool reverse, int columns, const PassParams& p, const StripParams& s, cudaStream_t stream);
+cudaError_t launch_strips(bool reverse, bool aa, int columns, const PassParams& p, const StripParams& s, int blocks,
+                          cudaStream_t stream);
 
 }  // namespace gbsw
