@@ -192,9 +192,9 @@ bool fits_int8(int v) { return v >= -127 && v <= 127; }
 // * DNA: one pair per 32-lane group up to about 10,000 pairs; above that two
 //   pairs per group (the dual-pair kernel) in the narrowest group that still
 //   gets 2.5 two-pair units, i.e. pairs x lanes >= 5 x `lanes`: 4 lanes from
-//   ~97,000 pairs, 8 from ~49,000, else 16.  On the DNA throughput shapes at
-//   25,000 pairs: 2.57 ms at 16 lanes, 3.25 at 8, 5.38 at 4; at 50,000: 4.41 at
-//   8, 5.75 at 4; at 100,000: 8.05 at 4 or 8, 8.59 at 16.
+//   ~97,000 pairs, 8 from ~49,000, else 16.  On the DNA throughput shapes both
+//   passes at 20,000 pairs: 1.50 ms at 16 lanes, 1.46 at 8, 1.80 at 4; at 50,000:
+//   3.58, 3.17 and 3.01; at 100,000: 7.04, 5.99 and 5.63.
 // * Protein (log-normal lengths up to 1,000): one pair per 32-lane group up to
 //   about 10 waves of pairs, and two pairs per 16-lane group above (1.5x faster
 //   than one pair at 60,000-120,000 pairs, slower below 24,000).
@@ -483,18 +483,23 @@ int run_passes(gbsw_context* ctx, const gbsw_scoring* sc, const uint8_t* ref, co
         gbsw_variant v = table.variant[sc->kind][b][count_bucket(count)];
         gbsw_variant rv = table.reverse[sc->kind][b][count_bucket(count)];
         if (!use_table || count <= 0 || !variant_ok(protein, v, dual_ok)) return;
-        // Pairs of at most 512 symbols end soon even two to a group: 8,000 reads of
-        // 100-150 against 200-500 bp take 271 us forward so and 281 strip by strip, 4,000
-        // 258 and 177 (longer pairs: 8,000 of the throughput shape 875 and 604).
-        if (ctx->tuning_builtin && !protein && b == 0 && !v.dual && v.lanes == gbsw::kTeamLanes && count > 7000 &&
-            max_len <= 512)
-            v = rv = gbsw_variant{1, 16};
-        // A few long proteins among many short ones: one launch over both bins ends
-        // sooner once the short ones fill it (60,000 pairs, 6,215 of them long: 7.38
-        // against 7.68 ms for both passes; 34,000 pairs: 5.21 against 4.60).
+        // Pairs of at most 1,024 symbols end soon even two to a group: 8,000 of the throughput
+        // shape take 533 + 244 us (both passes) so and 579 + 336 strip by strip, 5,000 454 + 223
+        // and 387 + 219.
+        const bool strips_dna = ctx->tuning_builtin && !protein && !v.dual && v.lanes == gbsw::kTeamLanes;
+        if (strips_dna && b == 0 && count > 6000 && max_len <= 1024) v = rv = gbsw_variant{1, 16};
+        // Long pairs' reverse pass, where bands leave little work: 5,919 of the mixed shape
+        // take 2.8 ms in groups and 3.6 strip by strip, 1,469 2.0 and 1.0.
+        if (strips_dna && b == 1 && count > 4500) rv = gbsw_variant{1, 16};
+        // A few long proteins among many short ones: one launch over both bins ends sooner
+        // once the short ones fill it, forward 25,000 pairs 1.40 against 1.56 ms (15,000: a
+        // long pair's own 0.94 against 0.75), reverse 45,000 pairs 2.01 against 2.15 (30,000:
+        // 1.78 against 1.51).
         if (ctx->tuning_builtin && protein && b == 1 && !v.dual && v.lanes == gbsw::kTeamLanes &&
-            plan.bin[0][0].dual && ctx->stats.bin_pairs[0] > 50000)
-            v = rv = plan.bin[0][0];
+            plan.bin[0][0].dual) {
+            if (ctx->stats.bin_pairs[0] > 20000) v = plan.bin[0][0];
+            if (ctx->stats.bin_pairs[0] > 35000) rv = plan.bin[1][0];
+        }
         plan.bin[0][b] = plan.bin[1][b] = v;
         if (variant_ok(protein, rv, dual_ok)) plan.bin[1][b] = rv;
         plan.from_table[b] = true;

@@ -22,8 +22,9 @@ cudaError_t launch_pass(int score, bool reverse, bool dpx, int width, const Pass
                         cudaStream_t stream);
 // Kernel of a wide variant (sw_wide.cu), nullptr if none.
 const void* pick_wide(int width, int score, bool reverse);
-// Dual-pair int16x2 passes (class kClassDual), sw_dual.cu: DNA at width 4,
-// protein (`aa`) at widths 16 and 32.  has_dual tells whether a variant exists.
+// Dual-pair int16x2 passes, sw_dual.cu: DNA at widths 4, 8 and 16 (run with twice the
+// lanes of 8 columns), protein (`aa`) at widths 16 and 32.  has_dual tells whether a
+// variant exists.
 bool has_dual(bool aa, int width);
 // Lanes per group of the dual variant a plan of `width` runs (sizes its scratch).
 int dual_lanes(bool aa, int width);

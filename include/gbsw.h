@@ -238,7 +238,8 @@ int gbsw_last_stats(const gbsw_context* ctx, gbsw_stats* stats);
  * whose matrix fits int8, with gap values in [-16384, 0] -- fall into two length
  * bins by their shorter sequence: below 512, and from 512 up.  Each bin is its
  * own launch with its own variant, in each pass: two pairs per lane group in
- * the int16x2 kernels (dual = 1; DNA at 4, 8 or 16 lanes, protein at 16 or 32)
+ * the int16x2 kernels (dual = 1; DNA at 4, 8 or 16 lanes, which name strips of 64,
+ * 128 and 256 columns, protein at 16 or 32)
  * or one pair per group in int32 (dual = 0; 4, 8, 16 or 32 lanes, or 128: block
  * per pair).  With lane_group = 0 the call reads the bins' pair counts back
  * after the forward schedule (one small copy and a wait on the stream) and takes
