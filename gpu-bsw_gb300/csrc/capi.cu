@@ -431,6 +431,15 @@ int run_passes(gbsw_context* ctx, const gbsw_scoring* sc, const uint8_t* ref, co
     auto wide_strips = [&](int64_t long_pairs) {
         return !protein && max_len >= gbsw::kLongCols && strip_tasks(long_pairs, 4) >= 8192;
     };
+    // The table's entry.  3,000 to 10,000 long proteins run two to a group in a batch whose
+    // short ones fill the GPU beside them (25,000 pairs: forward 1.40 against 1.56 ms strip
+    // by strip), and strip by strip in a smaller one, which ends with its longest pair
+    // (15,000: 0.94 against 0.75).
+    auto table_entry = [&](int rev, int b, int bucket) {
+        if (ctx->tuning_builtin && protein && !rev && b == 1 && bucket == 2 && n <= 24000)
+            return gbsw_variant{0, gbsw::kTeamLanes};
+        return (rev ? table.reverse : table.variant)[sc->kind][b][bucket];
+    };
     // A small batch whose plan is block per pair whatever its bins hold: one block
     // schedules it, and nothing waits for the counts (unless they choose the strips'
     // width).
@@ -442,8 +451,8 @@ int run_passes(gbsw_context* ctx, const gbsw_scoring* sc, const uint8_t* ref, co
             continue;
         }
         for (int k = 0; small && k <= count_bucket(n); ++k) {
-            const gbsw_variant& rv = table.reverse[sc->kind][b][k];
-            small = team(table.variant[sc->kind][b][k]) && (team(rv) || !variant_ok(protein, rv, dual_ok));
+            const gbsw_variant rv = table_entry(1, b, k);
+            small = team(table_entry(0, b, k)) && (team(rv) || !variant_ok(protein, rv, dual_ok));
         }
     }
     gbsw::StripParams strip_params{};
@@ -480,8 +489,8 @@ int run_passes(gbsw_context* ctx, const gbsw_scoring* sc, const uint8_t* ref, co
     // the device too, and the other ranges launch whatever they hold.
     auto take_count = [&](int b, int64_t count) {
         ctx->stats.bin_pairs[b] = count;
-        gbsw_variant v = table.variant[sc->kind][b][count_bucket(count)];
-        gbsw_variant rv = table.reverse[sc->kind][b][count_bucket(count)];
+        gbsw_variant v = table_entry(0, b, count_bucket(count));
+        gbsw_variant rv = table_entry(1, b, count_bucket(count));
         if (!use_table || count <= 0 || !variant_ok(protein, v, dual_ok)) return;
         // Pairs of at most 1,024 symbols end soon even two to a group: 8,000 of the throughput
         // shape take 533 + 244 us (both passes) so and 579 + 336 strip by strip, 5,000 454 + 223
@@ -491,14 +500,12 @@ int run_passes(gbsw_context* ctx, const gbsw_scoring* sc, const uint8_t* ref, co
         // Long pairs' reverse pass, where bands leave little work: 5,919 of the mixed shape
         // take 2.8 ms in groups and 3.6 strip by strip, 1,469 2.0 and 1.0.
         if (strips_dna && b == 1 && count > 4500) rv = gbsw_variant{1, 16};
-        // A few long proteins among many short ones: one launch over both bins ends sooner
-        // once the short ones fill it, forward 25,000 pairs 1.40 against 1.56 ms (15,000: a
-        // long pair's own 0.94 against 0.75), reverse 45,000 pairs 2.01 against 2.15 (30,000:
-        // 1.78 against 1.51).
-        if (ctx->tuning_builtin && protein && b == 1 && !v.dual && v.lanes == gbsw::kTeamLanes &&
-            plan.bin[0][0].dual) {
-            if (ctx->stats.bin_pairs[0] > 20000) v = plan.bin[0][0];
-            if (ctx->stats.bin_pairs[0] > 35000) rv = plan.bin[1][0];
+        // Long proteins among many short ones: one launch over both bins ends sooner once
+        // the short ones fill it (reverse 45,000 pairs 2.01 against 2.15 ms, 30,000 1.78
+        // against 1.51).
+        if (ctx->tuning_builtin && protein && b == 1 && plan.bin[0][0].dual && ctx->stats.bin_pairs[0] > 35000) {
+            if (!v.dual && v.lanes == gbsw::kTeamLanes) v = plan.bin[0][0];
+            if (!rv.dual && rv.lanes == gbsw::kTeamLanes) rv = plan.bin[1][0];
         }
         plan.bin[0][b] = plan.bin[1][b] = v;
         if (variant_ok(protein, rv, dual_ok)) plan.bin[1][b] = rv;

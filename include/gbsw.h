@@ -250,7 +250,8 @@ int gbsw_last_stats(const gbsw_context* ctx, gbsw_stats* stats);
  * entry with lanes = 0 leaves the bin to the rule of gbsw_options.lane_group =
  * 0 (the batch size picks one width; long DNA pairs of a 4-lane plan run 16-lane
  * dual groups).  A context starts with a table measured on GB300 by
- * gpu-bsw_gb300/tune_sweep.py.
+ * gpu-bsw_gb300/tune_sweep.py; while it stands, a few counts within a bucket take
+ * another variant than the bucket's entry (gbsw_last_stats reports the one that ran).
  */
 typedef struct {
     int32_t dual;   /* 1: two pairs per group, int16x2; 0: one pair per group, int32 */
