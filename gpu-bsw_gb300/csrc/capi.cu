@@ -810,6 +810,11 @@ int decode_device_error(gbsw_context* ctx, int flags) {
 // paths' walks (100,000 DNA pairs in three launches 1.28 ms of walks, in one 0.57).
 constexpr int64_t kTraceBudget = int64_t(1) << 30;
 constexpr int64_t kTraceBudgetFree = int64_t(5) << 30;
+// DNA calls of this many pairs run their bands in small groups, one pair after another;
+// fewer end sooner with a pair's strips spread over warps (kernels, banded against strips:
+// 7,000 throughput pairs 0.55 and 0.46 ms, 20,000 0.66 and 1.01; 6,000 mixed ones 5.04 and
+// 3.03, 20,000 5.28 and 9.17).
+constexpr int64_t kBandPairs = 12000;
 
 int traceback_host(gbsw_context* ctx, const gbsw_scoring* sc, const char* ref, const int64_t* ref_off,
                    const char* query, const int64_t* query_off, int64_t n, const int32_t* top_scores,
@@ -849,6 +854,14 @@ int traceback_host(gbsw_context* ctx, const gbsw_scoring* sc, const char* ref, c
     auto fits16 = [&](int m, int kk, int score) {
         return scores16 && gbsw::trace16_pair_ok(lim16, m, kk, score, sc->gap_open, sc->gap_extend);
     };
+    // Many DNA pairs at a time: their bands, in small groups.
+    const bool many = !protein && scores16 && n >= kBandPairs;
+    auto banded = [&](int m, int kk) {
+        return many && gbsw::band_pair_ok(sc->match, sc->mismatch, m, kk, sc->gap_open, sc->gap_extend);
+    };
+    auto band_of = [&](int m, int kk, int score) {
+        return gbsw::trace_band_of(m, kk, score, sc->match, sc->gap_open, sc->gap_extend);
+    };
     // per pair: operation slot (m + k), direction words and boundary entries of
     // its launch; launches cut where the budget fills
     e = ctx->h_tb_off.reserve((size_t)5 * n + 1);
@@ -856,10 +869,10 @@ int traceback_host(gbsw_context* ctx, const gbsw_scoring* sc, const char* ref, c
     int64_t* slot = ctx->h_tb_off.ptr;       // n + 1
     int64_t* dir_off = slot + n + 1;         // n
     int64_t* bnd_off = dir_off + n;          // n
-    int64_t* order = slot + 4 * n + 1;       // n: each launch's pairs by descending cost, int16 ones first
+    int64_t* order = slot + 4 * n + 1;       // n: each launch's pairs by descending cost, banded ones, int16 ones, the others
     std::vector<int64_t> cuts{0};
     int64_t dir_max = 1, bnd_max = 1, dir_run = 0, bnd_run = 0, total_tasks = 0, total_bytes = 0;
-    int rows16 = 1;  // largest row count (k + 1) of an int16 pair
+    int rows16 = 1, band_rows = 0;  // largest row counts (k + 1) of the int16 pairs, strip by strip and banded
     slot[0] = 0;
     for (int64_t k = 0; k < n; ++k) {
         int64_t cap = 0, dw = 0, bw = 0;
@@ -870,7 +883,11 @@ int traceback_host(gbsw_context* ctx, const gbsw_scoring* sc, const char* ref, c
                 return ctx->fail(GBSW_EINVAL, "traceback: begins/ends out of range for pair " + std::to_string(k));
             const int m = ref_end[k] - ref_begin[k], kk = query_end[k] - query_begin[k];
             cap = (int64_t)m + kk;
-            if (fits16(m, kk, top_scores[k])) {
+            if (banded(m, kk)) {
+                dw = gbsw::band_strip_words(band_of(m, kk, top_scores[k]), kk) *
+                     ((m + gbsw::kBandWidth - 1) / gbsw::kBandWidth);
+                band_rows = std::max(band_rows, kk + 1);
+            } else if (fits16(m, kk, top_scores[k])) {
                 dw = gbsw::trace16_dir_words(m, kk);
                 total_tasks += (m + gbsw::kTrace16Width - 1) / gbsw::kTrace16Width;
                 rows16 = std::max(rows16, kk + 1);
@@ -908,11 +925,12 @@ int traceback_host(gbsw_context* ctx, const gbsw_scoring* sc, const char* ref, c
     }
     cuts.push_back(n);
     // Each launch's pairs by descending row steps (int16: strips x (row pairs + fill),
-    // int32: strips x (rows + fill)), so that the pairs a warp's groups or walks run
+    // banded over the band's, int32: strips x (rows + fill)), so that the pairs a warp's groups or walks run
     // together end close together: a counting sort over 8 buckets per doubling of
     // the cost (the exponent and the next three bits of the integer cost).
     const size_t launches = cuts.size() - 1;
-    std::vector<int64_t> count16(launches), first_task(launches + 1);  // per launch: int16 pairs, their tasks
+    std::vector<int64_t> count_band(launches), count16(launches), first_task(launches + 1);  // per launch: banded
+                                                                   // and other int16 pairs, their tasks
     int64_t max_tasks = 0;
     e = ctx->h_tb_tasks.reserve((size_t)std::max<int64_t>(total_tasks, 1));
     if (e != cudaSuccess) return ctx->fail(GBSW_ENOMEM, "cudaMallocHost");
@@ -920,36 +938,38 @@ int traceback_host(gbsw_context* ctx, const gbsw_scoring* sc, const char* ref, c
         constexpr int kCostBuckets = 8 * 64;
         std::vector<uint16_t> bucket((size_t)n);
         for (int64_t k = 0; k < n; ++k) {
-            int b = 0, wide = 0;
+            int b = 0, kind = 1;  // 0: banded, 1: int16 (and no path), 2: int32
             if (top_scores[k] > 0) {
                 const int m = ref_end[k] - ref_begin[k], kk = query_end[k] - query_begin[k];
-                wide = fits16(m, kk, top_scores[k]) ? 0 : 1;
-                const uint64_t cost = wide ? (uint64_t)((m + gbsw::kTraceCols - 1) / gbsw::kTraceCols) *
-                                                 (uint64_t)(kk + gbsw::kTraceLanes - 1)
-                                           : (uint64_t)((m + gbsw::kTrace16Width - 1) / gbsw::kTrace16Width) *
-                                                 (uint64_t)(kk / 2 + 64);
+                kind = banded(m, kk) ? 0 : fits16(m, kk, top_scores[k]) ? 1 : 2;
+                const auto strips = [&](int width) { return (uint64_t)((m + width - 1) / width); };
+                const uint64_t cost =
+                    kind == 0   ? strips(gbsw::kBandWidth) * (uint64_t)gbsw::band_strip_words(band_of(m, kk, top_scores[k]), kk)
+                    : kind == 1 ? strips(gbsw::kTrace16Width) * (uint64_t)(kk / 2 + 64)
+                                : strips(gbsw::kTraceCols) * (uint64_t)(kk + gbsw::kTraceLanes - 1);
                 const int e = 63 - __builtin_clzll(cost | 1);
                 const int frac = e >= 3 ? (int)((cost >> (e - 3)) & 7) : (int)((cost << (3 - e)) & 7);
                 b = std::min(kCostBuckets - 1, 1 + 8 * e + frac);
             }
-            bucket[(size_t)k] = (uint16_t)(wide * kCostBuckets + kCostBuckets - 1 - b);  // descending cost first
+            bucket[(size_t)k] = (uint16_t)(kind * kCostBuckets + kCostBuckets - 1 - b);  // descending cost first
         }
-        std::vector<int64_t> count(2 * kCostBuckets);
+        std::vector<int64_t> count(3 * kCostBuckets);
         int2* tasks = ctx->h_tb_tasks.ptr;
         int64_t nt = 0;
         for (size_t c = 0; c < launches; ++c) {
             std::fill(count.begin(), count.end(), 0);
             for (int64_t k = cuts[c]; k < cuts[c + 1]; ++k) ++count[bucket[(size_t)k]];
             int64_t at = cuts[c];
-            for (int b = 0; b < 2 * kCostBuckets; ++b) {
-                if (b == kCostBuckets) count16[c] = at - cuts[c];
+            for (int b = 0; b < 3 * kCostBuckets; ++b) {
+                if (b == kCostBuckets) count_band[c] = at - cuts[c];
+                if (b == 2 * kCostBuckets) count16[c] = at - cuts[c] - count_band[c];
                 const int64_t here = count[b];
                 count[b] = at;
                 at += here;
             }
             for (int64_t k = cuts[c]; k < cuts[c + 1]; ++k) order[count[bucket[(size_t)k]]++] = k;
             first_task[c] = nt;
-            for (int64_t x = cuts[c]; x < cuts[c] + count16[c]; ++x) {
+            for (int64_t x = cuts[c] + count_band[c]; x < cuts[c] + count_band[c] + count16[c]; ++x) {
                 const int64_t k = order[x];
                 if (top_scores[k] <= 0) continue;
                 const int strips = (ref_end[k] - ref_begin[k] + gbsw::kTrace16Width - 1) / gbsw::kTrace16Width;
@@ -979,6 +999,15 @@ int traceback_host(gbsw_context* ctx, const gbsw_scoring* sc, const char* ref, c
     if (max_tasks > 0) {
         rc = reserve_strips(ctx, max_tasks, total_tasks, rows16, stream, &strip_params);
         if (rc != GBSW_OK) return rc;
+    }
+    int band_blocks = 0;
+    band_rows = (band_rows + 1) & ~1;
+    if (band_rows > 0) {
+        e = gbsw::band_occupancy(&band_blocks);
+        if (e != cudaSuccess) return ctx->cuda_fail(e, "occupancy");
+        band_blocks = ctx->sms * std::max(1, band_blocks);
+        e = ctx->d_scratch.reserve((size_t)gbsw::band_groups(band_blocks) * (size_t)(band_rows / 2));
+        if (e != cudaSuccess) return ctx->fail(GBSW_ENOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
     }
     e = ctx->h_tb_count.reserve((size_t)n);
     if (e == cudaSuccess) e = ctx->h_misc.reserve(16);
@@ -1057,6 +1086,16 @@ int traceback_host(gbsw_context* ctx, const gbsw_scoring* sc, const char* ref, c
         tp.dir_off = d_off + (n + 1) + cuts[c];
         tp.bnd_off = d_off + (2 * n + 1) + cuts[c];
         tp.order = d_off + (4 * n + 1) + cuts[c];
+        tp.count = count_band[c];
+        if (tp.count > 0) {
+            e = cudaMemsetAsync(tp.queue, 0, sizeof(int), stream);
+            if (e == cudaSuccess)
+                e = gbsw::launch_trace_band(tp, reinterpret_cast<uint2*>(ctx->d_scratch.ptr), band_rows,
+                                            band_blocks, stream);
+            if (e != cudaSuccess) return ctx->cuda_fail(e, "traceback launch");
+            ctx->stats.launches += 2;
+        }
+        tp.order += count_band[c];
         tp.count = count16[c];
         if (ntasks > 0) {
             // the queue and the counters of blocks by SM
@@ -1072,7 +1111,7 @@ int traceback_host(gbsw_context* ctx, const gbsw_scoring* sc, const char* ref, c
         if (e != cudaSuccess) return ctx->cuda_fail(e, "traceback launch");
         ctx->stats.launches += (ntasks > 0) + (tp.count > 0);
         tp.order += count16[c];
-        tp.count = cuts[c + 1] - cuts[c] - count16[c];
+        tp.count = cuts[c + 1] - cuts[c] - count_band[c] - count16[c];
         ctx->stats.launches += tp.count > 0;
         e = gbsw::launch_trace(tp, stream);
         if (e != cudaSuccess) return ctx->cuda_fail(e, "traceback launch");

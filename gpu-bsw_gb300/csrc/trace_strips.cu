@@ -28,6 +28,8 @@
 // as the passes.  Row 0 and those before it are below every real value whatever
 // they add, and no real cell depends on rows and columns outside the pair.
 //
+// Calls of many DNA pairs run trace_band below, the same cells within a band.
+//
 // What bounds it: the DP, the ALU pipe (9 ALU and 8 other operations a cell pair,
 // where the int32 kernel spent 17 ALU operations on one cell); the walk, a
 // chain of one direction word per cell.
@@ -48,6 +50,42 @@ constexpr int kSymShift = 7;
 constexpr unsigned kRowPad = 0x7f;
 
 __device__ __forceinline__ int gap_cost(int open, int ext, int len) { return open + (len - 1) * ext; }
+
+// Two rows of a lane's columns, both halves: the row above in hup (H), hop (H + open) and
+// fup (F), H(i-1, left) in diag0, H and E of the left edge's two rows in h_in and e (E:
+// on to the right neighbour); leaves the rows' H in first and hup and their direction bits.
+template <class Score>
+__device__ __forceinline__ void two_rows(unsigned (&hup)[kTrace16Cols], unsigned (&hop)[kTrace16Cols],
+                                         unsigned (&fup)[kTrace16Cols], unsigned diag0, const unsigned (&h_in)[2],
+                                         unsigned (&e)[2], unsigned open2, unsigned ext2, Score score,
+                                         unsigned (&first)[kTrace16Cols], unsigned& bits_ef, unsigned& bits_h) {
+    unsigned diag[2] = {diag0, h_in[0]}, left[2] = {__vadd2(h_in[0], open2), __vadd2(h_in[1], open2)};
+#pragma unroll
+    for (int c = 0; c < kTrace16Cols; ++c) {
+        unsigned up = hup[c], upo = hop[c], f = fup[c];
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const unsigned d = __vadd2(diag[r], score(r, c));
+            const unsigned ee = __vadd2(e[r], ext2), fe = __vadd2(f, ext2);
+            e[r] = __vmaxs2(ee, left[r]);  // E(i, j)
+            f = __vmaxs2(fe, upo);         // F(i, j)
+            const unsigned h = __vimax3_s16x2(d, f, e[r]);
+            // signs: E opened, F opened; F < H, diagonal < H
+            const unsigned ef = prmt(__vsub2(ee, left[r]), __vsub2(fe, upo), 0xFDB9u);
+            const unsigned hh = prmt(__vsub2(f, h), __vsub2(d, h), 0xFDB9u);
+            const unsigned bit = 0x01010101u << (4 * r + c);
+            bits_ef |= ef & bit;
+            bits_h |= hh & bit;
+            diag[r] = up;
+            up = h;
+            upo = left[r] = __vadd2(h, open2);
+            if (r == 0) first[c] = h;
+        }
+        hup[c] = up;
+        hop[c] = upo;
+        fup[c] = f;
+    }
+}
 
 template <bool PROTEIN>
 __global__ void __launch_bounds__(kThreads, 4) trace_strips(TraceParams p, StripParams s, int ntasks) {
@@ -202,37 +240,14 @@ __global__ void __launch_bounds__(kThreads, 4) trace_strips(TraceParams p, Strip
                         wb[r] = *reinterpret_cast<const unsigned*>(prof + kAAProfRows * kResidue + (code[r] >> 16));
                     }
                 }
-                unsigned diag[2] = {diag0, h_in[0]}, left[2] = {__vadd2(h_in[0], open2), __vadd2(h_in[1], open2)};
                 unsigned first[C], bits_ef = 0, bits_h = 0;
-#pragma unroll
-                for (int c = 0; c < C; ++c) {
-                    unsigned up = hup[c], upo = hop[c], f = fup[c];
-#pragma unroll
-                    for (int r = 0; r < 2; ++r) {
-                        unsigned d;
-                        if constexpr (PROTEIN)
-                            d = __vadd2(diag[r], prmt(wa[r], wb[r], (unsigned)c * 0x1111u + 0xC480u));
-                        else
-                            d = __vadd2(diag[r], __viaddmax_s16x2(~(code[r] ^ rc[c]), match_up, mismatch2));
-                        const unsigned ee = __vadd2(e[r], ext2), fe = __vadd2(f, ext2);
-                        e[r] = __vmaxs2(ee, left[r]);                    // E(i, j)
-                        f = __vmaxs2(fe, upo);                           // F(i, j)
-                        const unsigned h = __vimax3_s16x2(d, f, e[r]);
-                        // signs: E opened, F opened; F < H, diagonal < H
-                        const unsigned ef = prmt(__vsub2(ee, left[r]), __vsub2(fe, upo), 0xFDB9u);
-                        const unsigned hh = prmt(__vsub2(f, h), __vsub2(d, h), 0xFDB9u);
-                        const unsigned bit = 0x01010101u << (4 * r + c);
-                        bits_ef |= ef & bit;
-                        bits_h |= hh & bit;
-                        diag[r] = up;
-                        up = h;
-                        upo = left[r] = __vadd2(h, open2);
-                        if (r == 0) first[c] = h;
-                    }
-                    hup[c] = up;
-                    hop[c] = upo;
-                    fup[c] = f;
-                }
+                two_rows(
+                    hup, hop, fup, diag0, h_in, e, open2, ext2,
+                    [&](int r, int c) -> unsigned {
+                        if constexpr (PROTEIN) return prmt(wa[r], wb[r], (unsigned)c * 0x1111u + 0xC480u);
+                        else return __viaddmax_s16x2(~(code[r] ^ rc[c]), match_up, mismatch2);
+                    },
+                    first, bits_ef, bits_h);
 #pragma unroll
                 for (int r = 0; r < 2; ++r) x_e[r] = __shfl_sync(kFull, e[r], src);
                 x_h[0] = __shfl_sync(kFull, first[C - 1], src);
@@ -272,6 +287,196 @@ __global__ void __launch_bounds__(kThreads, 4) trace_strips(TraceParams p, Strip
     }
 }
 
+// The DP of DNA pairs whose score leaves their paths a narrow band (trace_band_of), many
+// pairs at a time: groups of 4 lanes take pairs from the queue and run a pair's strips
+// (8 virtual lanes, 32 columns) one after another, over the band's rows only.  A cell
+// outside the band counts as -inf.  That leaves every cell of every path of the pair's
+// score as it was, a candidate that ties with one among them, and no cell above its
+// value, so the walk meets the same choices; a score that is not the segment's gives a
+// path value that differs from it, as without a band.  The strip's edge goes through a
+// buffer of the group's own, a word a row, in place: rows are read a chunk before they
+// are written.
+//
+// A read of 225 symbols at the throughput shape's error rate keeps 2 x 21 diagonals
+// of its 225 rows.  In 256-column strips of a whole warp it took 169 steps of a warp,
+// two thirds of their cells outside the segment or the band; here 7 strips of 46 steps
+// of an eighth of one.  100,000 such pairs, DP and walks: 4.71 -> 1.67 ms, with 1.8 in
+// place of 4.3 GB of directions.  Bound by the ALU pipe, as the strips.
+__global__ void __launch_bounds__(kThreads, 4) trace_band(TraceParams p, uint2* edges, int rows) {
+    constexpr int C = kTrace16Cols, G = kBandLanes, W = kBandWidth, kGroups = kThreads / G;
+    constexpr int kFetch = kTraceSteps / G;  // row pairs a lane fetches for a chunk
+    static_assert(kTraceSteps % G == 0 && kThreads == 128, "the fetch and band_groups");
+    // what lane 0 takes in at each step: the edge words of its two rows, their codes
+    __shared__ __align__(16) uint4 sin_[kGroups][2][kTraceSteps];
+    const int lane = threadIdx.x & 31, g = lane % G, grp = threadIdx.x / G;
+    const unsigned gmask = ((1u << G) - 1u) << (lane - g);
+    const int src = lane - g + (g + G - 1) % G;
+    // lane 0: the injected word's low (or high) half, then lane G - 1's low half
+    const unsigned sel_lo = g ? 0x3210u : 0x1054u, sel_hi = g ? 0x3210u : 0x1076u;
+    const int open = p.open, ext = p.ext;
+    const unsigned open2 = pack16(open, open), ext2 = pack16(ext, ext), neg2 = pack16(kBandNeg, kBandNeg);
+    const unsigned match_up = pack16(p.match + 1, p.match + 1), mismatch2 = pack16(p.mismatch, p.mismatch);
+    uint2* const edge = edges + ((size_t)blockIdx.x * kGroups + grp) * (size_t)(rows / 2);
+
+    // ---- group state ----
+    bool busy = false, done = false;
+    int pid = 0, m = 0, k = 0, strip = 0, t = 0, t_end = 0, buf = 0;
+    int p0 = 0, p1 = -1, have = -1;  // the strip's first and last row pair, the last one its left edge holds
+    int keep_end = 0, t_fin = -1, vm = 0, hand_on = 0;  // hand_on: row pairs whose edge the next strip reads
+    TraceBand band{0, 0};
+    const uint8_t *R = p.ref, *Q = p.query;
+    uint2* dir = nullptr;
+    // ---- lane state ----
+    unsigned hup[C], hop[C], fup[C], rc[C];
+    unsigned diag0 = neg2, x_h[2] = {neg2, neg2}, x_e[2] = {neg2, neg2}, x_code[2] = {0, 0};
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+        hup[c] = hop[c] = fup[c] = neg2;
+        rc[c] = 0;
+    }
+
+    auto row_code = [&](int i) -> unsigned {
+        return i >= 1 && i <= k ? (unsigned)Q[i - 1] << kSymShift : kRowPad;
+    };
+    uint2 nedge[kFetch];
+    unsigned ncode[kFetch];
+    auto issue = [&](int t0) {  // lane g: row pairs g, g + G of the chunk
+#pragma unroll
+        for (int x = 0; x < kFetch; ++x) {
+            const int q = p0 + t0 + g + x * G, i = 2 * q;
+            ncode[x] = row_code(i) | (row_code(i + 1) << 16);
+            if (strip > 0) {
+                nedge[x] = q <= have ? __ldcg(edge + q) : make_uint2(neg2, neg2);
+            } else {
+                nedge[x].x = pack16(i <= k ? (i > 0 ? gap_cost(open, ext, i) : 0) : kBandNeg, kBandNeg);
+                nedge[x].y = pack16(i < k ? gap_cost(open, ext, i + 1) : kBandNeg, kBandNeg);
+            }
+        }
+    };
+    auto commit = [&](int b) {
+#pragma unroll
+        for (int x = 0; x < kFetch; ++x)
+            sin_[grp][b][g + x * G] = make_uint4(nedge[x].x, nedge[x].y, ncode[x], 0);
+    };
+    auto setup_strip = [&] {
+        const int lanes = min(2 * G, (m - strip * W + C - 1) / C);
+        const bool last = (strip + 1) * W >= m;
+        have = p1;
+        p0 = band_first_pair(band, strip);
+        p1 = band_last_pair(band, strip, k);
+        const int pairs = p1 - p0 + 1;
+        t = 0;
+        t_end = pairs + lanes - 1;
+        keep_end = g < lanes ? min(t_end, g + pairs + (lanes > G ? G : 0)) : 0;
+        vm = ((m - 1) % W) / C;
+        t_fin = last ? (k >> 1) - p0 + vm : -1;
+        hand_on = last ? 0 : pairs;
+        const int j_a = strip * W + g * C + 1, j_b = j_a + G * C;  // first columns (1-based) of the halves
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+            rc[c] = ((j_a + c <= m ? (unsigned)R[j_a + c - 1] : 0u) |
+                     ((j_b + c <= m ? (unsigned)R[j_b + c - 1] : 0u) << 16)) << kSymShift;
+            hup[c] = fup[c] = neg2;
+            hop[c] = pack16(kBandNeg + open, kBandNeg + open);
+        }
+        diag0 = x_h[0] = x_h[1] = x_e[0] = x_e[1] = neg2;
+        x_code[0] = x_code[1] = kRowPad * 0x10001u;  // rows before the strip's
+        buf = 0;
+        issue(0);
+        commit(0);
+    };
+
+    while (true) {
+        if (!done && !busy) {
+            int at = 0;
+            if (g == 0) at = atomicAdd(p.queue, 1);
+            at = __shfl_sync(gmask, at, lane - g);
+            if (at >= p.count) {
+                done = true;
+                keep_end = hand_on = 0;
+                t_fin = -1;
+            } else {
+                pid = (int)p.order[at];
+                const int score = p.score[pid];
+                if (score > 0) {
+                    const int rb = p.ref_begin[pid], qb = p.query_begin[pid];
+                    m = p.ref_end[pid] - rb;
+                    k = p.query_end[pid] - qb;
+                    R = p.ref + p.ref_off[pid] + rb;
+                    Q = p.query + p.query_off[pid] + qb;
+                    band = trace_band_of(m, k, score, p.match, open, ext);
+                    dir = reinterpret_cast<uint2*>(p.dir + p.dir_off[pid - p.first]);
+                    strip = 0;
+                    p1 = -1;
+                    busy = true;
+                    setup_strip();
+                }
+            }
+            __syncwarp(gmask);
+        }
+        if (__all_sync(kFull, done)) break;
+        if (__any_sync(kFull, !done && !busy)) continue;  // a pair without a path: take the next one
+
+        // ---- kTraceSteps steps, every lane of the warp ----
+        if (busy) issue(t + kTraceSteps);
+        uint4 next = sin_[grp][buf][0];  // loaded a step ahead
+        uint2 kept[4];
+#pragma unroll 4
+        for (int u = 0; u < kTraceSteps; ++u) {
+            const uint4 in = next;
+            next = sin_[grp][buf][(u + 1) % kTraceSteps];
+            const unsigned code[2] = {prmt(x_code[0], in.z, sel_lo), prmt(x_code[1], in.z, sel_hi)};
+            x_code[0] = __shfl_sync(kFull, code[0], src);
+            x_code[1] = __shfl_sync(kFull, code[1], src);
+            const unsigned h_in[2] = {prmt(x_h[0], in.x, sel_lo), prmt(x_h[1], in.y, sel_lo)};
+            unsigned e[2] = {prmt(x_e[0], in.x, sel_hi), prmt(x_e[1], in.y, sel_hi)};
+            unsigned first[C], bits_ef = 0, bits_h = 0;
+            two_rows(
+                hup, hop, fup, diag0, h_in, e, open2, ext2,
+                [&](int r, int c) { return __viaddmax_s16x2(~(code[r] ^ rc[c]), match_up, mismatch2); }, first,
+                bits_ef, bits_h);
+#pragma unroll
+            for (int r = 0; r < 2; ++r) x_e[r] = __shfl_sync(kFull, e[r], src);
+            x_h[0] = __shfl_sync(kFull, first[C - 1], src);
+            x_h[1] = __shfl_sync(kFull, hup[C - 1], src);
+            diag0 = h_in[1];
+            kept[u % 4] = make_uint2(bits_ef, bits_h);
+            if (u % 4 == 3 && t >= g && t - 3 < keep_end) {
+                uint4* const at = reinterpret_cast<uint4*>(dir + (t >> 2) * (4 * G) + 4 * g);
+                at[0] = make_uint4(kept[0].x, kept[0].y, kept[1].x, kept[1].y);
+                at[1] = make_uint4(kept[2].x, kept[2].y, kept[3].x, kept[3].y);
+            }
+            const int q = t - (2 * G - 1);  // the last virtual lane's row pair
+            if (g == G - 1 && (unsigned)q < (unsigned)hand_on)
+                __stcg(edge + p0 + q, make_uint2(prmt(first[C - 1], e[0], 0x7632u), prmt(hup[C - 1], e[1], 0x7632u)));
+            if (t == t_fin) {
+                unsigned h = 0;
+#pragma unroll
+                for (int c = 0; c < C; ++c)
+                    if (c == (m - 1) % C) h = (k & 1) ? hup[c] : first[c];
+                if (g == vm % G) p.path_score[pid] = vm >= G ? hi16(h) : lo16(h);
+            }
+            ++t;
+        }
+        if (busy && t < t_end) {
+            buf ^= 1;
+            commit(buf);
+        } else if (busy) {
+            __syncwarp(gmask);  // this strip's edge before the next one reads it
+            if ((strip + 1) * W < m) {
+                dir += band_strip_words(band, k) / 2;
+                ++strip;
+                setup_strip();
+            } else {
+                busy = false;
+                keep_end = hand_on = 0;
+                t_fin = -1;
+            }
+        }
+        __syncwarp();
+    }
+}
+
 // The paths of the launch's pairs, in the order of their cost (a warp's walks end
 // close together), a group of kWalkLanes lanes each.  The lanes walk in step, so
 // that each of them can fetch a part of what comes next: a tile holds, for the
@@ -281,8 +486,10 @@ __global__ void __launch_bounds__(kThreads, 4) trace_strips(TraceParams p, Strip
 // next one.  (One thread per pair took 0.92 ms for the walks of 7,001 proteins, most
 // of it in one of 32 lanes' misses at every step.)  Runs are written from the
 // slot's end backwards, which leaves them in path order.
+template <bool BAND>
 __global__ void __launch_bounds__(kWalkThreads) walk_paths(TraceParams p) {
     constexpr int L = kWalkLanes, S = 4 * L;  // symbols of a tile
+    constexpr int G = BAND ? kBandLanes : 32, W = BAND ? kBandWidth : kTrace16Width;
     __shared__ __align__(16) uint4 s_dir[kWalkThreads / L][L][4];
     __shared__ uint8_t s_r[kWalkThreads / L][S], s_q[kWalkThreads / L][S];
     const int lane = threadIdx.x & 31, g = lane % L, grp = threadIdx.x / L;
@@ -307,11 +514,12 @@ __global__ void __launch_bounds__(kWalkThreads) walk_paths(TraceParams p) {
     const uint8_t* const R = p.ref + p.ref_off[pid] + rb;
     const uint8_t* const Q = p.query + p.query_off[pid] + qb;
     const uint4* const dir = reinterpret_cast<const uint4*>(p.dir + p.dir_off[pid - p.first]);
-    const int pairs = (k + 2) / 2;
-    const int64_t per_strip = trace16_strip_words(pairs, 64) / 4;
+    TraceBand band{0, 0};
+    if constexpr (BAND) band = trace_band_of(m, k, score, p.match, p.open, p.ext);
+    const int64_t per_strip = (BAND ? band_strip_words(band, k) : trace16_strip_words((k + 2) / 2, 64)) / 4;
     uint32_t* out = p.ops + p.slot_off[pid + 1];
     int i = k, j = m, state = 0, n = 0;
-    int ti = 0, tj = 0, tv = -1, tt = 0;  // the tile's first cell, its virtual lane (-1: no tile) and first step
+    int ti = 0, tj = 0, tv = 0, tt = 0, ts = -1;  // the tile's first cell, its virtual lane, first step and strip (-1: no tile)
     uint32_t run = 0;  // the run being extended (len << 4 | op)
     auto push = [&](uint32_t op) {
         if ((run & 15u) == op) {
@@ -326,28 +534,30 @@ __global__ void __launch_bounds__(kWalkThreads) walk_paths(TraceParams p) {
         }
     };
     while (i > 0 && j > 0) {
-        const int c = (j - 1) % kTrace16Width, v = c / kTrace16Cols, t = (i >> 1) + v;
+        const int strip = (j - 1) / W, c = (j - 1) % W, v = c / kTrace16Cols;
+        const int p0 = BAND ? band_first_pair(band, strip) : 0, t = (i >> 1) - p0 + v;
         int l = tv - v;
         // of the two sectors the tile holds for virtual lane tv - l, step / 4 of the second
         int sector = (t >> 2) - ((tt - 3 * l) >> 2) + 1;
-        if ((unsigned)l >= (unsigned)L || (unsigned)sector > 1u || (unsigned)((ti - i) | (tj - j)) >= (unsigned)S) {
+        if (strip != ts || (unsigned)l >= (unsigned)L || (unsigned)sector > 1u || (unsigned)((ti - i) | (tj - j)) >= (unsigned)S) {
             ti = i;
             tj = j;
             tv = v;
+            ts = strip;
             l = 0;
             // the diagonal enters the columns of virtual lane v - l in row first - 4 l, so
             // in step tt - 1 - 3 l
-            tt = ((i + 3 - c % kTrace16Cols) >> 1) + v + 1;
+            tt = ((i + 3 - c % kTrace16Cols) >> 1) - p0 + v + 1;
             sector = (t >> 2) - (tt >> 2) + 1;
             __syncwarp(gmask);  // every lane is done with the old tile
-            const int strip = (j - 1) / kTrace16Width;
-            const int lanes = min(64, (m - strip * kTrace16Width + kTrace16Cols - 1) / kTrace16Cols);
+            const int lanes = min(2 * G, (m - strip * W + kTrace16Cols - 1) / kTrace16Cols);
+            const int pairs = (BAND ? band_last_pair(band, strip, k) : k >> 1) - p0 + 1;
             const int last_q = (pairs + lanes - 2) >> 2, q = (tt - 3 * g) >> 2;  // the strip's last step / 4
             if (v - g >= 0) {
-                const uint4* const src = dir + (int64_t)strip * per_strip + (int64_t)q * 64 + 2 * ((v - g) & 31);
+                const uint4* const src = dir + (int64_t)strip * per_strip + (int64_t)q * (2 * G) + 2 * ((v - g) % G);
                 if (q >= 1 && q - 1 <= last_q) {
-                    s_dir[grp][g][0] = src[-64];
-                    s_dir[grp][g][1] = src[-63];
+                    s_dir[grp][g][0] = src[-2 * G];
+                    s_dir[grp][g][1] = src[-2 * G + 1];
                 }
                 if (q >= 0 && q <= last_q) {
                     s_dir[grp][g][2] = src[0];
@@ -363,7 +573,7 @@ __global__ void __launch_bounds__(kWalkThreads) walk_paths(TraceParams p) {
         }
         const bool same = s_r[grp][tj - j] == s_q[grp][ti - i];
         const uint2 w = reinterpret_cast<const uint2*>(s_dir[grp][l])[4 * sector + (t & 3)];
-        const int sh = (v >= 32 ? 8 : 0) + 4 * (i & 1) + c % kTrace16Cols;
+        const int sh = (v >= G ? 8 : 0) + 4 * (i & 1) + c % kTrace16Cols;
         if (state == 0) {
             if (!((w.y >> (16 + sh)) & 1u)) {
                 push(same ? kOpEq : kOpX);
@@ -394,6 +604,13 @@ __global__ void __launch_bounds__(kWalkThreads) walk_paths(TraceParams p) {
 
 }  // namespace
 
+namespace {
+unsigned walk_blocks(int64_t pairs) {
+    constexpr int kPerBlock = kWalkThreads / kWalkLanes;
+    return (unsigned)((pairs + kPerBlock - 1) / kPerBlock);
+}
+}  // namespace
+
 cudaError_t trace16_occupancy(bool protein, int* blocks_per_sm) {
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(
         blocks_per_sm, protein ? (const void*)trace_strips<true> : (const void*)trace_strips<false>, kThreads, 0);
@@ -409,8 +626,20 @@ cudaError_t launch_trace16(const TraceParams& p, const StripParams& s, int ntask
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
-    constexpr int kPerBlock = kWalkThreads / kWalkLanes;
-    walk_paths<<<(unsigned)((p.count + kPerBlock - 1) / kPerBlock), kWalkThreads, 0, stream>>>(p);
+    walk_paths<false><<<walk_blocks(p.count), kWalkThreads, 0, stream>>>(p);
+    return cudaGetLastError();
+}
+
+cudaError_t band_occupancy(int* blocks_per_sm) {
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, (const void*)trace_band, kThreads, 0);
+}
+
+cudaError_t launch_trace_band(const TraceParams& p, uint2* edges, int rows, int blocks, cudaStream_t stream) {
+    if (p.count <= 0) return cudaSuccess;
+    trace_band<<<blocks, kThreads, 0, stream>>>(p, edges, rows);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    walk_paths<true><<<walk_blocks(p.count), kWalkThreads, 0, stream>>>(p);
     return cudaGetLastError();
 }
 

@@ -114,6 +114,52 @@ inline int64_t trace16_dir_words(int m, int k) {
     const int lanes = (m - (strips - 1) * kTrace16Width + kTrace16Cols - 1) / kTrace16Cols;
     return (strips - 1) * trace16_strip_words(pairs, 64) + trace16_strip_words(pairs, lanes);
 }
+// ---- its banded form for many DNA pairs (trace_band in trace_strips.cu) ----
+// Lanes of a group, columns of its strips (two virtual lanes of 4 columns a lane).
+constexpr int kBandLanes = 4;
+constexpr int kBandWidth = 2 * kBandLanes * kTrace16Cols;
+constexpr int kBandMaxRows = 2048;  // a group's edge buffer holds a word a row
+constexpr int kBandNeg = -14000;    // its -inf
+// Whether a pair's segment suits it: real values within 12,000 of 0 on both sides, so
+// that the difference of any two values, -inf's among them, fits 16 bits (a value below
+// -inf has lost at most 16 for each of the 39 rows and columns of a strip and its fill).
+inline bool band_pair_ok(int match, int mismatch, int m, int k, int open, int ext) {
+    const int64_t both = m < k ? m : k;
+    return match > 0 && k < kBandMaxRows && m < kBandMaxRows && match * both <= 12000 &&
+           (mismatch < 0 ? mismatch : 0) * both + 2 * (int64_t)open + (int64_t)ext * ((int64_t)m + k) >= -12000;
+}
+// The diagonals i - j that a path of this score can visit.  A path that leaves those
+// between (0, 0) and (k, m) by d has d gap symbols more on both sides and d aligned
+// pairs less: match (min(m, k) - d) + 2 open + (|m - k| + 2 d - 2) ext at best.
+struct TraceBand {
+    int lo, hi;
+};
+__host__ __device__ inline TraceBand trace_band_of(int m, int k, int score, int match, int open, int ext) {
+    const int both = m < k ? m : k, apart = m < k ? k - m : m - k;
+    const int64_t spare = (int64_t)(match * both + 2 * open + (apart - 2) * ext) - score;
+    const int d = spare > 0 ? (int)spare / (match - 2 * ext) : 0;
+    return {(k < m ? k - m : 0) - d, (k > m ? k - m : 0) + d};
+}
+// First and last row pair of a strip, and its direction words (two per lane and step,
+// steps rounded up to four), the same for every strip of the pair.
+__host__ __device__ inline int band_first_pair(const TraceBand& b, int strip) {
+    const int i = strip * kBandWidth + b.lo;
+    return (i > 0 ? i : 0) >> 1;
+}
+__host__ __device__ inline int band_last_pair(const TraceBand& b, int strip, int k) {
+    const int i = strip * kBandWidth + kBandWidth + b.hi;
+    return (i < k ? i : k) >> 1;
+}
+__host__ __device__ inline int64_t band_strip_words(const TraceBand& b, int k) {
+    const int all = (k >> 1) + 1, most = (kBandWidth + b.hi - b.lo) / 2 + 2, pairs = all < most ? all : most;
+    return (int64_t)((pairs + 2 * kBandLanes - 1 + 3) / 4) * (8 * kBandLanes);
+}
+cudaError_t band_occupancy(int* blocks_per_sm);
+inline int band_groups(int blocks) { return blocks * (128 / kBandLanes); }
+// The DP of the pairs p.order[0 .. p.count) in `blocks` blocks (p.queue 0 before the
+// launch; `edges`: `rows` / 2 entries per group, rows even and above every k), then
+// their walks.
+cudaError_t launch_trace_band(const TraceParams& p, uint2* edges, int rows, int blocks, cudaStream_t stream);
 cudaError_t trace16_occupancy(bool protein, int* blocks_per_sm);
 // The DP of `ntasks` strip tasks (s.tasks, a pair's strips one after another), then
 // the walks of the pairs p.order[0 .. p.count), their runs at the ends of their slots.
