@@ -21,7 +21,7 @@ NVCC = os.environ.get("NVCC", shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVCC_FLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-O2",
                      "-I" + INCLUDE, "-I" + CSRC] + os.environ.get("GBSW_NVCC_FLAGS", "").split()
-GBSW_SOURCES = ["sw_kernels.cu", "sw_wide.cu", "sw_dual.cu", "sw_strips.cu", "traceback.cu", "trace_strips.cu", "schedule.cu", "capi.cu", "calib.cu",
+GBSW_SOURCES = ["sw_kernels.cu", "sw_wide.cu", "sw_dual.cu", "sw_bound.cu", "sw_strips.cu", "traceback.cu", "trace_strips.cu", "schedule.cu", "capi.cu", "calib.cu",
                 "noalloc.cu", "unpack.cu", "pack.cpp", "driver.cpp",
                 "pinned_pool.cpp",
                 "server.cpp"]

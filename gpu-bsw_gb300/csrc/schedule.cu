@@ -47,6 +47,19 @@ __device__ __forceinline__ int dual_bucket(int nrows, int ncols) {
 }
 static_assert(64 * 128 <= kBinBuckets, "dual keys");
 
+// DNA forward passes with score bounds: the rows a unit computes are those that either
+// half's bound leaves, so that pairs without one come first and the others by the place
+// of their diagonal, in 7 steps, within a group of like width and rows (short bin 64
+// columns and 32 rows, long bin 128 and 128).
+__device__ __forceinline__ int bound_bucket(bool is_short, int nrows, int ncols, int2 bound) {
+    const int spare = nrows - ncols + 1;
+    const int place = bound.x <= 0 ? 7 : min(6, max(0, bound.y) * 7 / spare);
+    const int strips = is_short ? min(7, (ncols - 1) / 64) : min(31, (ncols - 1) / 128);
+    const int rows = is_short ? min(127, nrows / 32) : min(31, nrows / 128);
+    return kBinBuckets - 1 - ((((strips << (is_short ? 7 : 5)) | rows) << 3) | place);
+}
+static_assert(8 * 128 * 8 <= kBinBuckets && 32 * 32 * 8 <= kBinBuckets && kLongCols <= 512, "bound keys");
+
 // Key of a pair of class `cls` (its entry of the per-pair class array): the
 // bins share class kClassBinned, long bin first.  `fine`: the DNA reverse keys.
 __device__ __forceinline__ int pair_key(int cls, int nrows, int ncols, bool fine = false) {
@@ -123,7 +136,10 @@ __global__ void forward_keys(SchedParams s) {
             // units and is longest-first for one-pair plans as well
             s.cls[k] = (uint8_t)cls;
             if (s.classes_only) continue;
-            const int key = pair_key(cls, nrows, ncols);
+            const int key = s.bound && is_bin_class(cls) && ncols > 0
+                                ? class_base(kClassBinned) + (cls == kClassShort ? kBinBuckets : 0) +
+                                      bound_bucket(cls == kClassShort, nrows, ncols, s.bound[k])
+                                : pair_key(cls, nrows, ncols);
             s.keys[k] = key;
             atomicAdd(&s.hist[key], 1);
         }

@@ -30,6 +30,7 @@ struct SchedParams {
     int* class_range;     // 2 * kRanges ints: [begin, end) of each class, then of the two bins
     int* order;           // n pair indices in schedule order
     int* error;
+    const int2* bound;    // forward keys: score bounds (sw_bound.cu), which order like diagonals (nullptr: none)
     int classes_only;     // forward keys: write the classes and nothing else
 };
 

@@ -126,6 +126,9 @@ struct PassParams {
     int dual_limit;
     int* rerun;
     uint8_t* pair_cls;
+    // Dual-pair forward pass: per pair, the score of some alignment of it (0: none known) and
+    // the difference of its rows and columns (nullptr: no bounds)
+    const int2* bound;
     // 1: this launch runs beside the one before it (launch_beside), and ends after it
     int join;
 };

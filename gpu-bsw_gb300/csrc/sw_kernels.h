@@ -22,6 +22,9 @@ cudaError_t launch_pass(int score, bool reverse, bool dpx, int width, const Pass
                         cudaStream_t stream);
 // Kernel of a wide variant (sw_wide.cu), nullptr if none.
 const void* pick_wide(int width, int score, bool reverse);
+// Lower bounds of the scores of A/C/G/T pairs (sw_bound.cu; those of others mean nothing),
+// and the diagonals (row - column) they lie on; match > 0.
+cudaError_t launch_score_bounds(const PassParams& p, int2* bound, int sms, cudaStream_t stream);
 // Dual-pair int16x2 passes, sw_dual.cu: DNA at widths 4, 8 and 16 (run with twice the
 // lanes of 8 columns), protein (`aa`) at widths 16 and 32.  has_dual tells whether a
 // variant exists.
