@@ -76,7 +76,7 @@ AA_GAPS = (-6, -1)
 # DRAM bytes (read + write) of one forward launch, from an ncu capture of this
 # workload (dram__bytes_read.sum + dram__bytes_write.sum); the algorithmic input
 # is the sequences and offsets, about 95 MB for the default batch
-TRAFFIC = {"dna_throughput": 430.4e6 + 542.2e6, "protein": 21.5e6 + 1.1e6}
+TRAFFIC = {"dna_throughput": 142.1e6 + 167.7e6, "protein": 21.1e6 + 1.0e6}
 # workload -> (pairs, seed, kind, description); the default is the headline batch
 WORKLOADS = {
     "dna_throughput": (100_000, 2, "dna", "refs U[400,1024] bp, queries U[150,300] bp, 80% mutated substrings"),
@@ -401,7 +401,11 @@ def roofline(cells, fwd_ms, dual, lane_group, calib, mhz, traffic=None):
     pair of the dual kernel is 6.5 int16x2 ops, all on the integer ALU pipe,
     which takes a warp instruction every other cycle per SM sub-partition (64
     lane-ops per clock per SM); an int32 cell is 6.5 ops, some of which issue to
-    other pipes, so its bound is the issue rate (128 lane-ops per clock per SM)."""
+    other pipes, so its bound is the issue rate (128 lane-ops per clock per SM).
+
+    `cells` are the matrices': rows that the forward pass leaves out by score bounds
+    (large DNA batches) count as done, so the fraction is of work asked for, not of
+    cells computed, and the kernel itself issues 5.5 of the probe's 6.5 ops to the pipe."""
     peak_cal = calib["cell_dual_gcups"] if dual else calib["cell_int32_gcups"]
     ops_per_cell = 3.25 if dual else 6.5
     lane_ops = 64 if dual else 128
