@@ -68,7 +68,7 @@
 // reverse_low_band): a unit's strips start and end at the rows its wider band needs, and
 // both halves compute every row between.
 //
-// Score bounds (BOUND, DNA forward): with a score F that the pair is known to reach
+// Score bounds (LIVE, DNA forward): with a score F that the pair is known to reach
 // (sw_bound.cu, or the best of the strips before), a strip need only compute rows that an
 // alignment scoring F or more can visit.  From a row of the left edge whose H lies below
 // F - match x (the columns from there on), no alignment reaches F: the others are live.
@@ -78,7 +78,11 @@
 // out count as empty ones, which only lowers cells that no such alignment visits, so the
 // best cells, all of them, stay.  A unit computes the rows of both halves, and the schedule
 // brings together pairs with like diagonals.  100,000 reads, four of five related: forward
-// 4.19 -> 3.70 ms without that order, with it 3.26; long pairs of the mixed shape 55.7 -> 45.
+// 4.19 -> 3.70 ms without that order, with it 3.26; long pairs of the mixed shape 55.7 -> 39.
+// The reverse pass (LIVE) knows its score.  Its alignments begin in the first column
+// (reverse_band), so that none begins in a later strip, and a row of a strip's edge is live
+// if its H and match x (the rows from there on) reach the score: of the band, which has
+// the same width in every strip, that leaves half.
 //
 // Measured, 100,000 reads against contigs (8 lanes): forward 4.65 -> 4.19 ms, reverse
 // (16 lanes) 1.92 -> 1.49 against one row of 16 columns a step with a row test in every
@@ -145,7 +149,7 @@ constexpr size_t dual_smem() {
     return dual_row_bytes<REVERSE, AA, G, C>() + (AA ? (size_t)2 * kAAProfRows * kThreads * C : 0);
 }
 
-template <bool REVERSE, bool BOUND>
+template <bool REVERSE, bool LIVE>
 __device__ __forceinline__ void load_half(const PassParams& p, Half& h, int pid) {
     h = Half{};
     h.pid = pid;
@@ -167,7 +171,7 @@ __device__ __forceinline__ void load_half(const PassParams& p, Half& h, int pid)
         h.rowseq = h.a_short ? B : A;
         h.ncols = h.ncols_run = h.a_short ? a : b;
         h.nrows = h.a_short ? b : a;
-        if (BOUND) h.floor = min(p.bound[pid].x, p.dual_limit);
+        if (LIVE) h.floor = min(p.bound[pid].x, p.dual_limit);
     } else {
         const int target = p.score[pid];
         const int na = p.ref_end[pid], nb = p.query_end[pid];
@@ -188,13 +192,13 @@ __device__ __forceinline__ void load_half(const PassParams& p, Half& h, int pid)
     }
 }
 
-template <bool REVERSE, bool BOUND>
+template <bool REVERSE, bool LIVE>
 __device__ __forceinline__ void write_half(const PassParams& p, const Half& h, uint64_t best) {
     const int pid = h.pid;
     if (pid < 0) return;
     if constexpr (!REVERSE) {
         const int v = (int)(best >> 32);
-        if (BOUND && v < h.floor) atomicOr(p.error, kErrNoHit);
+        if (LIVE && v < h.floor) atomicOr(p.error, kErrNoHit);
         if (v > p.dual_limit) {  // may have wrapped in int16: rerun in int32
             p.rerun[2 + atomicAdd(p.rerun + 1, 1)] = pid;
             p.pair_cls[pid] = 0;
@@ -224,7 +228,7 @@ __device__ __forceinline__ void write_half(const PassParams& p, const Half& h, u
     }
 }
 
-template <bool REVERSE, bool AA, int G, int C, bool BOUND>
+template <bool REVERSE, bool AA, int G, int C, bool LIVE>
 __global__ void __launch_bounds__(kThreads, REVERSE && !AA ? 5 : 4) sw_pass_dual(PassParams p) {
     let_next_start();
     constexpr int W = G * C, kGroups = kThreads / G;
@@ -243,8 +247,8 @@ __global__ void __launch_bounds__(kThreads, REVERSE && !AA ? 5 : 4) sw_pass_dual
     __shared__ unsigned s_floor[kThreads];
     // forward: the Ho from which a row of this strip's edge is live (both halves), and the
     // rows of the next strip that live ones reach
-    __shared__ unsigned s_thr[BOUND ? kGroups : 1];
-    __shared__ int2 s_live[BOUND ? kGroups : 1];
+    __shared__ unsigned s_thr[LIVE && !REVERSE ? kGroups : 1];
+    __shared__ int2 s_live[LIVE ? kGroups : 1];
     __shared__ uint64_t s_best[2][kThreads];
     extern __shared__ __align__(16) unsigned char sdyn[];
     int4(*const srow)[C / 4][kThreads] = reinterpret_cast<int4(*)[C / 4][kThreads]>(sdyn);
@@ -280,7 +284,7 @@ __global__ void __launch_bounds__(kThreads, REVERSE && !AA ? 5 : 4) sw_pass_dual
     int nstrips = 0, strip = 0, t = 0, t_end = 0, buf = 0;
     int nrows = 0;      // the taller pair's rows
     int have = 0;       // rows the previous strip's edge holds
-    int last_rows = 0;  // forward: the previous strip's last row
+    int last_rows = 0;  // live rows: the previous strip's last row
     int write_rows = 0; // rows whose edge goes to the next strip (0: last strip)
     // ---- lane state ----
     unsigned ho[C], f[C], pa[AA ? 1 : C], pb[AA ? 1 : C];
@@ -398,21 +402,39 @@ __global__ void __launch_bounds__(kThreads, REVERSE && !AA ? 5 : 4) sw_pass_dual
             const int band = unit_band(half[0], half[1]), low = unit_low_band(half[0], half[1]);
             last_row = band_last_row(strip * W + W, low, nrows);
             have = band_last_row(strip * W, low, nrows);
-            t = (min(band_first_row(strip * W + 1, band), last_row) - 1) / 2;  // the band's first row is odd
+            int first_row = min(band_first_row(strip * W + 1, band), last_row);
+            if constexpr (LIVE) {
+                if (strip > 0) {
+                    first_row = max(first_row, s_live[grp].x);
+                    last_row = min(last_row, s_live[grp].y);
+                    have = last_rows;
+                }
+                last_rows = last_row;
+                if (!last_strip) {
+                    // halves without a band may begin an alignment in any strip
+                    int2 live = make_int2(nrows + 1, 0);
+#pragma unroll
+                    for (int x = 0; x < 2; ++x)
+                        if (half[x].nrows > 0 && half[x].band < 0) live = make_int2(1, max(live.y, half[x].nrows));
+                    __syncwarp(gmask);  // s_live is read
+                    if (g == 0) s_live[grp] = live;
+                }
+            }
+            t = (first_row - 1) / 2;
             lanes = min(G, (max(half[0].ncols_run, half[1].ncols_run) - strip * W + C - 1) / C);
             // one below the score a half looks for, which it so passes once
             mx = pack16(half[0].target > 0 ? half[0].target - 1 + open : 0x7fff,
                         half[1].target > 0 ? half[1].target - 1 + open : 0x7fff);
         } else {
-            have = BOUND ? last_rows : nrows;
+            have = LIVE ? last_rows : nrows;
             // lanes of padding only are the matrix boundary whatever the row
             t = strip == 0 ? min(half[0].pad, half[1].pad) / C : 0;
-            if (BOUND && strip > 0) {
+            if (LIVE && strip > 0) {
                 t = (s_live[grp].x - 1) / 2;
                 last_row = s_live[grp].y;
             }
             last_rows = last_row;
-            if (BOUND && !last_strip) {
+            if (LIVE && !last_strip) {
                 unsigned thr = 0;
                 int2 live = make_int2(nrows + 1, 0);
 #pragma unroll
@@ -501,12 +523,12 @@ __global__ void __launch_bounds__(kThreads, REVERSE && !AA ? 5 : 4) sw_pass_dual
                 if (g < 2) half[g].nrows = 0;  // the rest of the warp's chunks run on padding
                 __syncwarp(gmask);
             } else {
-                if (g < 2) load_half<REVERSE, BOUND>(p, half[g], k0 + g < qend ? p.order[k0 + g] : -1);
+                if (g < 2) load_half<REVERSE, LIVE>(p, half[g], k0 + g < qend ? p.order[k0 + g] : -1);
                 __syncwarp(gmask);
                 nrows = max(half[0].nrows, half[1].nrows);
                 nstrips = (max(half[0].ncols_run, half[1].ncols_run) + W - 1) / W;
                 if (nrows == 0 || nstrips == 0) {
-                    if (g < 2) write_half<REVERSE, BOUND>(p, half[g], REVERSE ? ~0ull : 0ull);
+                    if (g < 2) write_half<REVERSE, LIVE>(p, half[g], REVERSE ? ~0ull : 0ull);
                 } else {
                     // forward: left-padded; reverse: padded on the right, which keeps
                     // the band's first rows those of the real columns
@@ -515,7 +537,7 @@ __global__ void __launch_bounds__(kThreads, REVERSE && !AA ? 5 : 4) sw_pass_dual
                     __syncwarp(gmask);
                     strip = 0;
                     if constexpr (!REVERSE)
-                        mx = s_floor[threadIdx.x] = BOUND ? pack16(max(half[0].floor - 1, 0) + open, max(half[1].floor - 1, 0) + open) : open2;
+                        mx = s_floor[threadIdx.x] = LIVE ? pack16(max(half[0].floor - 1, 0) + open, max(half[1].floor - 1, 0) + open) : open2;
                     busy = true;
                     setup_strip();
                 }
@@ -621,18 +643,26 @@ __global__ void __launch_bounds__(kThreads, REVERSE && !AA ? 5 : 4) sw_pass_dual
             const int row = settle(1, t, grew_b, before);
             mi_b = row > 0 ? row : mi_b;
         }
-        if constexpr (BOUND) {
+        if constexpr (LIVE) {
             if (g == G - 1 && write_rows > 0) {
                 // Live rows among the chunk's: none of its edge values (E is at most H) lies
                 // further above its last row's H than a gap down to there costs.
-                const unsigned thr = s_thr[grp];
                 const int r0 = 2 * (t - g) + 1;  // the chunk's first row here
 #pragma unroll
                 for (int x = 0; x < 2; ++x) {
-                    const int over = (x ? hi16(ho[C - 1]) - hi16(thr) : lo16(ho[C - 1]) - lo16(thr)) -
-                                     (open + (kDualRows - 2) * ext);
-                    if (over >= 0) {
-                        const int each = -max(open, ext);  // a gap symbol's least cost
+                    int over = (x ? hi16(ho[C - 1]) : lo16(ho[C - 1])) - (open + (kDualRows - 2) * ext);
+                    int each = -max(open, ext);  // a gap symbol's least cost
+                    bool live_rows = true;
+                    if constexpr (REVERSE) {
+                        // the score must be reached over the rows that are left, and a gap takes some
+                        const int rows = half[x].nrows - r0 + 1;
+                        over += max_score * rows - half[x].target - open;
+                        each += max_score;
+                        live_rows = rows > 0 && half[x].band >= 0;
+                    } else {
+                        over -= x ? hi16(s_thr[grp]) : lo16(s_thr[grp]);
+                    }
+                    if (live_rows && over >= 0) {
                         const int reach = each > 0 ? over / each : nrows;
                         int2 live = s_live[grp];
                         live.x = min(live.x, max(r0, 1));
@@ -690,7 +720,7 @@ __global__ void __launch_bounds__(kThreads, REVERSE && !AA ? 5 : 4) sw_pass_dual
             }
             __syncwarp(gmask);  // this strip's edge before the next one reads it
             ++strip;
-            if (strip < nstrips && (!BOUND || s_live[grp].x <= s_live[grp].y)) {
+            if (strip < nstrips && (!LIVE || s_live[grp].x <= s_live[grp].y)) {
                 setup_strip();
             } else {
                 uint64_t a = s_best[0][threadIdx.x], b = s_best[1][threadIdx.x];
@@ -700,7 +730,7 @@ __global__ void __launch_bounds__(kThreads, REVERSE && !AA ? 5 : 4) sw_pass_dual
                     a = REVERSE ? (oa < a ? oa : a) : (oa > a ? oa : a);
                     b = REVERSE ? (ob < b ? ob : b) : (ob > b ? ob : b);
                 }
-                if (g < 2) write_half<REVERSE, BOUND>(p, half[g], g ? b : a);
+                if (g < 2) write_half<REVERSE, LIVE>(p, half[g], g ? b : a);
                 busy = false;
                 write_rows = 0;
             }
@@ -711,32 +741,32 @@ __global__ void __launch_bounds__(kThreads, REVERSE && !AA ? 5 : 4) sw_pass_dual
 }
 
 template <bool AA, int G, int C>
-const void* dual_pass(bool reverse, bool bound, size_t* dyn) {
+const void* dual_pass(bool reverse, bool live, size_t* dyn) {
     *dyn = reverse ? dual_smem<true, AA, G, C>() : dual_smem<false, AA, G, C>();
-    if (reverse) return (const void*)sw_pass_dual<true, AA, G, C, false>;
-    if constexpr (!AA)
-        if (bound) return (const void*)sw_pass_dual<false, AA, G, C, true>;
-    return (const void*)sw_pass_dual<false, AA, G, C, false>;
+    if constexpr (!AA) {
+        if (live) return reverse ? (const void*)sw_pass_dual<true, AA, G, C, true> : (const void*)sw_pass_dual<false, AA, G, C, true>;
+    }
+    return reverse ? (const void*)sw_pass_dual<true, AA, G, C, false> : (const void*)sw_pass_dual<false, AA, G, C, false>;
 }
 
-// Kernel and dynamic shared memory of a dual variant (`bound`: with score bounds, DNA
-// forward); nullptr if none.  DNA widths name a strip of 16 columns a lane (64, 128, 256
+// Kernel and dynamic shared memory of a dual variant (`live`: DNA, live rows only);
+// nullptr if none.  DNA widths name a strip of 16 columns a lane (64, 128, 256
 // columns); the kernel runs it with twice the lanes of 8 columns.
-const void* pick_dual(bool reverse, bool aa, int width, bool bound, size_t* dyn) {
+const void* pick_dual(bool reverse, bool aa, int width, bool live, size_t* dyn) {
     *dyn = 0;
     if (!aa) {
-        if (width == 4) return dual_pass<false, 8, kDualCols>(reverse, bound, dyn);
-        if (width == 8) return dual_pass<false, 16, kDualCols>(reverse, bound, dyn);
-        if (width == 16) return dual_pass<false, 32, kDualCols>(reverse, bound, dyn);
+        if (width == 4) return dual_pass<false, 8, kDualCols>(reverse, live, dyn);
+        if (width == 8) return dual_pass<false, 16, kDualCols>(reverse, live, dyn);
+        if (width == 16) return dual_pass<false, 32, kDualCols>(reverse, live, dyn);
         return nullptr;
     }
-    if (width == 16) return dual_pass<true, 16, 8>(reverse, bound, dyn);
-    if (width == 32) return dual_pass<true, 32, 4>(reverse, bound, dyn);
+    if (width == 16) return dual_pass<true, 16, 8>(reverse, live, dyn);
+    if (width == 32) return dual_pass<true, 32, 4>(reverse, live, dyn);
     return nullptr;
 }
 
-cudaError_t prepare(bool reverse, bool aa, int width, bool bound, const void** fn, size_t* dyn) {
-    *fn = pick_dual(reverse, aa, width, bound, dyn);
+cudaError_t prepare(bool reverse, bool aa, int width, bool live, const void** fn, size_t* dyn) {
+    *fn = pick_dual(reverse, aa, width, live, dyn);
     if (!*fn) return cudaErrorInvalidValue;
     return cudaFuncSetAttribute(*fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*dyn);
 }
@@ -752,9 +782,12 @@ bool has_dual(bool aa, int width) {
 
 cudaError_t launch_pass_dual(bool reverse, bool aa, int width, const PassParams& p, int blocks,
                              cudaStream_t stream) {
+    // Reverse: where strips are many.  Long pairs of the mixed shape 18.4 -> 14.8 ms; 100,000
+    // reads 1.49 -> 1.56, 200,000 pairs of 100-150 against 200-500 symbols 1.16 -> 1.36.
+    const bool live = reverse ? p.cls == kRangeLong : p.bound != nullptr;
     size_t dyn = 0;
     const void* fn = nullptr;
-    cudaError_t e = prepare(reverse, aa, width, p.bound != nullptr, &fn, &dyn);
+    cudaError_t e = prepare(reverse, aa, width, live, &fn, &dyn);
     if (e != cudaSuccess) return e;
     void* args[] = {(void*)&p};
     return launch_beside(fn, blocks, kThreads, args, dyn, stream, p.join != 0);
