@@ -269,9 +269,9 @@ int dual_or_pass_occupancy(gbsw_context* ctx, bool protein, int score, bool rev,
 
 // DNA batches of this many pairs, some longer than kBoundLen, get score bounds before
 // their forward pass.  What the bounds cost (0.30 ms for 100,000 reads and references) comes
-// back where pairs are related: forward with them 4.29 -> 3.68 ms with four reads of five
-// related, 50,000 2.26 -> 2.16, 30,000 the same; 50,000 of the mixed shape 15.6 -> 13.3,
-// 20,000 7.3 -> 7.7.  (100,000 unrelated ones: 4.35 -> 4.61.)
+// back where pairs are related: forward with them 4.29 -> 3.65 ms with four reads of five
+// related, 40,000 1.90 -> 1.81, 30,000 1.56 -> 1.58; 50,000 of the mixed shape 15.8 -> 11.2,
+// 30,000 10.9 -> 12.1 (a long pair's chain of extensions).  (100,000 unrelated ones: 4.35 -> 4.61.)
 constexpr int64_t kBoundPairs = 40000;
 constexpr int kBoundLen = 512;
 

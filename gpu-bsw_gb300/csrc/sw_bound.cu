@@ -7,13 +7,15 @@
 // anchors of 12 symbols, evenly spaced over the shorter sequence, at every position of
 // the longer one.  The place of the anchor nearest to the middle is extended to both sides, a lane
 // each, 16 pairs at a time: along the diagonal while symbols agree, 16 at a step; where
-// two differ, on past them or past a gap of 1 to 3 on either side, whichever agrees
-// best over the 12 symbols behind it.  (On the throughput shape it finds the score itself
-// of half the related pairs, 95% of it on average.)
+// two differ, on past them or past a gap of 1 to 8 on either side, whichever agrees
+// best over the 10 symbols behind it.  (On the throughput shape it finds the score itself
+// of half the related pairs.)
 //
 // Bound by issue: a warp takes some 1,000 instructions to pack and scan a read and its
 // 700-symbol reference, and 300 for the next difference of 16 pairs.  100,000 of them: 0.30 ms
-// (a pair at a time, with 16 places extended each: 1.20).
+// (a pair at a time, with 16 places extended each: 1.20).  Gaps of 1 to 3 only lost the
+// alignment of one long pair in ten: forward pass of 200,000 mixed pairs 42.9 ms, with 1 to 5
+// 36, 1 to 8 32.9, 1 to 10 32.9.
 #include <algorithm>
 
 #include "strip_device.cuh"
@@ -23,13 +25,16 @@
 namespace gbsw {
 namespace {
 
-constexpr int kSeed = 12, kAnchors = 8;
+constexpr int kSeed = 12, kAnchors = 8, kGap = 8;  // symbols of a seed, seeds of a pair, longest gap of a step
+constexpr unsigned kBehindMask = (1u << 20) - 1;  // 10 symbols behind a difference
 constexpr unsigned kSeedMask = (1u << (2 * kSeed)) - 1;
 constexpr int kBoundRows = 8192, kBoundCols = 4096;  // longer pairs go without a bound
 // Smaller ones too: their few strips have little to leave out (140,000 reads of 100-150
 // against 300 symbols: forward 1.76 ms, with bounds 1.97).
 constexpr int kBoundCells = 1 << 16;
-constexpr int kBoundWords = 1024, kBoundPairs = 16;  // of a warp: packed words, pairs to extend
+// Of a warp: packed words, and in batches of longer pairs (200,000 mixed pairs, forward: 32.7
+// ms with 1,024 words, 31.3 with 4,096, 32.6 with 6,144), pairs to extend together.
+constexpr int kBoundWords = 1024, kBoundLongWords = 4096, kBoundPairs = 16;
 // A sequence's words and one past the last symbol's.
 __host__ __device__ constexpr int bound_words(int len) { return len / 16 + 2; }
 static_assert(bound_words(kBoundRows) + bound_words(kBoundCols) <= kBoundWords, "a pair fits");
@@ -99,12 +104,12 @@ __device__ int extend(const unsigned* rows, int nrows, const unsigned* cols, int
         // the symbols at (i, j) differ
         const unsigned r0 = window(rows, nrows, i, dir), c0 = window(cols, ncols, j, dir);
         auto gain = [&](unsigned a, unsigned b, int cost) {
-            return cost - __popc(differ(a, b) & kSeedMask) * step_off;
+            return cost - __popc(differ(a, b) & kBehindMask) * step_off;
         };
         int move_r = 1, move_c = 1, cost = p.mismatch;
         int top = gain(window(rows, nrows, i + dir, dir), window(cols, ncols, j + dir, dir), cost);
 #pragma unroll
-        for (int n = 1; n <= 3; ++n) {
+        for (int n = 1; n <= kGap; ++n) {
             const int gap = p.open + (n - 1) * p.ext;
             const int down = gain(window(rows, nrows, i + dir * n, dir), c0, gap);
             const int right = gain(r0, window(cols, ncols, j + dir * n, dir), gap);
@@ -134,11 +139,11 @@ struct BoundPair {
     int nrows, ncols, row, col;
 };
 
-__global__ void __launch_bounds__(kThreads) score_bounds(PassParams p, int2* bound) {
-    __shared__ unsigned s_words[kThreads / 32][kBoundWords];
+__global__ void __launch_bounds__(kThreads) score_bounds(PassParams p, int2* bound, int room) {
+    extern __shared__ unsigned s_words[];  // `room` a warp
     __shared__ BoundPair s_pair[kThreads / 32][kBoundPairs];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    unsigned* const words = s_words[warp];
+    unsigned* const words = s_words + warp * room;
     BoundPair* const pair = s_pair[warp];
     int used = 0, pairs = 0;
     auto extend_all = [&] {
@@ -166,7 +171,7 @@ __global__ void __launch_bounds__(kThreads) score_bounds(PassParams p, int2* bou
         if (lane == 0) bound[pid] = make_int2(0, 0);
         if (ncols < 2 * kSeed || (int64_t)nrows * ncols < kBoundCells || nrows >= kBoundRows || ncols >= kBoundCols) continue;
         const int need = bound_words(nrows) + bound_words(ncols);
-        if (pairs == kBoundPairs || used + need > kBoundWords) extend_all();
+        if (pairs == kBoundPairs || used + need > room) extend_all();
         unsigned *const rows = words + used, *const cols = rows + bound_words(nrows);
         const uint8_t *const ref_end = p.ref + p.ref_off[p.n], *const query_end = p.query + p.query_off[p.n];
         const bool flip = a < b;
@@ -207,7 +212,13 @@ __global__ void __launch_bounds__(kThreads) score_bounds(PassParams p, int2* bou
 
 cudaError_t launch_score_bounds(const PassParams& p, int2* bound, int sms, cudaStream_t stream) {
     const int64_t want = (p.n + kThreads / 32 - 1) / (kThreads / 32);
-    score_bounds<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)sms * 16)), kThreads, 0, stream>>>(p, bound);
+    const int room = p.scratch_rows > 1024 ? kBoundLongWords : kBoundWords;
+    const size_t dyn = (size_t)(kThreads / 32) * (size_t)room * sizeof(unsigned);
+    constexpr int kMost = kThreads / 32 * kBoundLongWords * (int)sizeof(unsigned);  // whatever other calls need
+    cudaError_t e = cudaFuncSetAttribute((const void*)score_bounds, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost);
+    if (e != cudaSuccess) return e;
+    const unsigned blocks = (unsigned)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)sms * 16));
+    score_bounds<<<blocks, kThreads, dyn, stream>>>(p, bound, room);
     return cudaGetLastError();
 }
 

@@ -78,7 +78,7 @@
 // out count as empty ones, which only lowers cells that no such alignment visits, so the
 // best cells, all of them, stay.  A unit computes the rows of both halves, and the schedule
 // brings together pairs with like diagonals.  100,000 reads, four of five related: forward
-// 4.19 -> 3.70 ms without that order, with it 3.26; long pairs of the mixed shape 55.7 -> 39.
+// 4.19 -> 3.70 ms without that order, with it 3.26; long pairs of the mixed shape 55.7 -> 27.
 // The reverse pass (LIVE) knows its score.  Its alignments begin in the first column
 // (reverse_band), so that none begins in a later strip, and a row of a strip's edge is live
 // if its H and match x (the rows from there on) reach the score: of the band, which has
